@@ -39,7 +39,7 @@ enum lg_status {
     LG_ERR_NOMEM = -3,     /* device allocation failed */
     LG_ERR_TIMEOUT = -4,   /* lg_sync gave up waiting */
     LG_ERR_STATE = -5,     /* call out of order (e.g. wrong dtype or field) */
-    LG_ERR_DEVICE = -6     /* a kernel reported a device-side error flag */
+    LG_ERR_DEVICE = -6     /* the device cannot run what was asked (a persistent kernel that does not fit) */
 };
 
 enum lg_dtype { LG_F64 = 0, LG_F32 = 1 };

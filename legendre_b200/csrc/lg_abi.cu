@@ -24,7 +24,6 @@ struct lg_ctx {
     std::string err;
     int64_t launches = 0;
     std::map<std::string, int> tuned;  // Model C variant chosen by lg_modelc_autotune, per shape
-    int* d_flag = nullptr;  // set by a kernel whose bounded device wait gave up (allocated on first use)
 };
 
 struct lg_grid {
@@ -235,16 +234,6 @@ int abi_state_view(const lg_state* st, StateView* v) {
     v->arena_rw = st->arena[st->cur];
     return LG_OK;
 }
-int* abi_device_flag(lg_ctx* ctx) {
-    if (!ctx->d_flag) {
-        if (cudaMalloc(&ctx->d_flag, sizeof(int)) != cudaSuccess) {
-            ctx->d_flag = nullptr;
-            return nullptr;
-        }
-        if (cudaMemsetAsync(ctx->d_flag, 0, sizeof(int), ctx->stream) != cudaSuccess) return nullptr;
-    }
-    return ctx->d_flag;
-}
 cudaStream_t abi_stream(lg_ctx* ctx) { return ctx->stream; }
 int abi_device(lg_ctx* ctx) { return ctx->device; }
 void abi_count_launch(lg_ctx* ctx, int64_t n) { ctx->launches += n; }
@@ -281,7 +270,6 @@ int lg_ctx_destroy(lg_ctx* ctx) {
     if (!ctx) return LG_ERR_INVALID;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
-    if (ctx->d_flag) cudaFree(ctx->d_flag);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return LG_OK;
@@ -291,22 +279,12 @@ const char* lg_last_error(const lg_ctx* ctx) { return ctx ? ctx->err.c_str() : "
 
 int64_t lg_ctx_kernel_launches(const lg_ctx* ctx) { return ctx ? ctx->launches : -1; }
 
-// after the stream has drained: did a kernel's bounded device wait give up?
-static int check_device_flag(lg_ctx* ctx) {
-    if (!ctx->d_flag) return LG_OK;
-    int v = 0;
-    LG_CUDA(ctx, cudaMemcpy(&v, ctx->d_flag, sizeof v, cudaMemcpyDeviceToHost));
-    if (v == 0) return LG_OK;
-    LG_CUDA(ctx, cudaMemset(ctx->d_flag, 0, sizeof(int)));
-    return fail(ctx, LG_ERR_DEVICE, "a kernel's bounded wait for its tile copies gave up; results are invalid");
-}
-
 int lg_sync(lg_ctx* ctx, int64_t timeout_ms) {
     if (!ctx) return LG_ERR_INVALID;
     auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t e = cudaStreamQuery(ctx->stream);
-        if (e == cudaSuccess) return check_device_flag(ctx);
+        if (e == cudaSuccess) return LG_OK;
         if (e != cudaErrorNotReady) return cuda_fail(ctx, e, "stream");
         if (timeout_ms >= 0) {
             auto ms = std::chrono::duration_cast<std::chrono::milliseconds>(std::chrono::steady_clock::now() - t0);
@@ -476,7 +454,7 @@ static int field_copy(lg_state* st, int field, void* host, int64_t nelem, bool u
                                        ctx->stream));
     }
     LG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-    return upload ? LG_OK : check_device_flag(ctx);
+    return LG_OK;
 }
 
 int lg_state_upload_field(lg_state* st, int field, const void* host, int64_t nelem) {
@@ -542,32 +520,33 @@ int lg_heat_fe_run(lg_state* st, int field, double kappa, double dt, int64_t nst
     const lg::SlabLayout L = layout_of(st, field);
     char key[256];
     snprintf(key, sizeof key, "heat|f=%d|k=%a|dt=%a", field, kappa, dt);
-    // 3-D: halos pulled from the neighbour blocks, ghosts filled once at the
-    // end; otherwise the push kernel, which keeps the ghosts valid each step
-    // (even block widths: the tiles staged by tensor copies; odd: by cp.async)
-    const bool pull = lg::heat3d_pull_supported(topo, L);
-    int* dflag = nullptr;
-    const bool tma = pull && lg::heat3d_tma_supported(topo, L) && (dflag = lg::abi_device_flag(ctx)) != nullptr;
-    auto step = [&]() -> int {
+    // 2-D and 3-D: two steps per launch, halos read from the neighbour blocks'
+    // interiors, ghosts filled once at the end; 1-D: the push kernel, one step
+    // per launch, which keeps the ghosts valid
+    const bool march = lg::heat_march_supported(topo, L);
+    auto launch = [&](int steps) -> int {
         const double* in = static_cast<const double*>(st->arena[st->cur]);
         double* out = static_cast<double*>(st->arena[st->cur ^ 1]);
-        cudaError_t e = tma    ? lg::launch_heat3d_tma(in, out, topo, L, field, kappa, dt, inv_h2, dflag, ctx->stream)
-                        : pull ? lg::launch_heat3d_pull(in, out, topo, L, field, kappa, dt, inv_h2, ctx->stream)
-                               : lg::launch_heat_step(in, out, topo, L, field, kappa, dt, inv_h2, ctx->stream);
+        cudaError_t e = march ? lg::launch_heat_march_fe(steps, in, out, topo, L, field, st->grid->periodic, kappa,
+                                                         dt, inv_h2, ctx->stream)
+                              : lg::launch_heat_step(in, out, topo, L, field, kappa, dt, inv_h2, ctx->stream);
         ctx->launches++;
         if (e != cudaSuccess) return cuda_fail(ctx, e, "heat step launch");
         st->cur ^= 1;
         st->tslot ^= 1;
         return LG_OK;
     };
-    int rc = run_steps(st, key, nsteps, flags, step);
+    // double steps, then single ones.  Fields that no launch writes keep to
+    // the arena the state began in: a state of several fields ends in the
+    // arena that one launch per step would leave it in
+    int64_t doubles = march ? nsteps / 2 : 0;
+    if (st->nfields > 1) doubles &= ~(int64_t)1;
+    int rc = run_steps(st, key + std::string("|2"), doubles, flags, [&] { return launch(2); });
+    if (rc == LG_OK) rc = run_steps(st, key, nsteps - 2 * doubles, flags, [&] { return launch(1); });
     if (rc != LG_OK) return rc;
-    if (pull && nsteps > 0) {
+    if (march && nsteps > 0) {
         rc = fill_all_ghosts(st);
         if (rc != LG_OK) return rc;
-    }
-    if (nsteps & 1) {
-        // graph replays keep parity; the remainder steps already flipped it
     }
     advance_time(st, dt, nsteps);
     return LG_OK;
@@ -827,11 +806,12 @@ int lg_modelc_initialize_grains(lg_state* st, const double* grains, int64_t n, d
     return lg_state_upload_field(st, 1, u.data(), (int64_t)u.size());
 }
 
-// the RungeKutta4 workspace: five arenas of the state's layout, zeroed
-static int rk_workspace(lg_state* st) {
-    if (st->rk[0]) return LG_OK;
+// the RungeKutta4 workspace: `n` arenas of the state's layout, zeroed
+static int rk_workspace(lg_state* st, int n) {
     const size_t bytes = (size_t)st->grid->nblocks * st->nfields * st->slab_stride * st->esize;
-    for (void*& q : st->rk) {
+    for (int i = 0; i < n; ++i) {
+        void*& q = st->rk[i];
+        if (q) continue;
         cudaError_t e = cudaMalloc(&q, bytes);
         if (e == cudaSuccess) e = cudaMemsetAsync(q, 0, bytes, st->ctx->stream);
         if (e != cudaSuccess) {
@@ -854,7 +834,10 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
         return fail(ctx, LG_ERR_STATE, "heat field must exist and have ghost width 1");
     if (nsteps < 0) return fail(ctx, LG_ERR_INVALID, "negative step count");
     cudaSetDevice(ctx->device);
-    int rc = rk_workspace(st);
+    const lg::CartTopo topo = topo_of(st->grid);
+    const lg::SlabLayout L = layout_of(st, field);
+    const bool march = lg::heat_march_supported(topo, L);
+    int rc = rk_workspace(st, march ? 2 : 5);
     if (rc != LG_OK) return rc;
     if (!st->ghosts_valid) {
         rc = fill_all_ghosts(st);
@@ -862,8 +845,6 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
     }
     double inv_h2[3] = {0, 0, 0};
     for (int d = 0; d < st->grid->D; ++d) inv_h2[d] = 1.0 / (st->grid->spacing[d] * st->grid->spacing[d]);
-    const lg::CartTopo topo = topo_of(st->grid);
-    const lg::SlabLayout L = layout_of(st, field);
     const double half_dt = 0.5 * dt, sixth = dt / 6.0, third = dt / 3.0;  // rk4.rs:57, 74-75
     char key[256];
     snprintf(key, sizeof key, "heat-rk4|f=%d|k=%a|dt=%a", field, kappa, dt);
@@ -875,7 +856,20 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
     auto step = [&]() -> int {
         const double* y = static_cast<const double*>(st->arena[st->cur]);
         double* out = static_cast<double*>(st->arena[st->cur ^ 1]);
-        cudaError_t e = lg::launch_heat_rk_stage(1, y, t0, y, k1, nullptr, nullptr, nullptr, topo, L, field, kappa,
+        cudaError_t e;
+        if (march) {  // 2-D and 3-D: two stages per launch, k1 and k2 hold y + c k2 and the running sum
+            e = lg::launch_heat_march_rk4(0, y, k1, nullptr, k2, topo, L, field, st->grid->periodic, kappa, dt,
+                                          inv_h2, ctx->stream);
+            if (e == cudaSuccess)
+                e = lg::launch_heat_march_rk4(1, k1, out, y, k2, topo, L, field, st->grid->periodic, kappa, dt,
+                                              inv_h2, ctx->stream);
+            ctx->launches += 2;
+            if (e != cudaSuccess) return cuda_fail(ctx, e, "heat RK4 launch");
+            st->cur ^= 1;
+            st->tslot ^= 1;
+            return LG_OK;
+        }
+        e = lg::launch_heat_rk_stage(1, y, t0, y, k1, nullptr, nullptr, nullptr, topo, L, field, kappa,
                                                  inv_h2, half_dt, 0.0, 0.0, ctx->stream);
         if (e == cudaSuccess)
             e = lg::launch_heat_rk_stage(1, t0, t1, y, k2, nullptr, nullptr, nullptr, topo, L, field, kappa, inv_h2,
@@ -893,6 +887,7 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
         return LG_OK;
     };
     rc = run_steps(st, key, nsteps, flags, step);
+    if (rc == LG_OK && march && nsteps > 0) rc = fill_all_ghosts(st);
     if (rc != LG_OK) return rc;
     advance_time(st, dt, nsteps);
     return LG_OK;
@@ -907,7 +902,7 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
         return fail(ctx, LG_ERR_INVALID, "RungeKutta4 steps deterministic models only (rk4.rs:15-19): noise must be 0");
     if (nsteps < 0) return fail(ctx, LG_ERR_INVALID, "negative step count");
     cudaSetDevice(ctx->device);
-    int rc = rk_workspace(st);
+    int rc = rk_workspace(st, 5);
     if (rc != LG_OK) return rc;
     if (!st->ghosts_valid) {
         rc = fill_all_ghosts(st);

@@ -32,24 +32,25 @@ cudaError_t launch_halo_fill(void* arena, int elem_size, const CartTopo& topo, c
                              cudaStream_t s);
 
 // (d) forward-Euler heat step: out = in + dt * (kappa * lap(in)) on the
-// interiors, plus the ghost ring of `out` filled from the new interiors.
+// interiors, plus the ghost ring of `out` filled from the new interiors.  1-D
+// grids (and dimensions of more than 2^30 cells); the others march (below).
 cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
                              double kappa, double dt, const double inv_h2[3], cudaStream_t s);
 
-// (d) the same heat step for 3-D grids of ghost width 1, with every halo
-// value read from the neighbour blocks' interiors: `out` gets interiors only
-// (its ghost entries are left as they were).  Bit-identical to
-// launch_heat_step.  Needs n0 * n1 <= 1024.
-bool heat3d_pull_supported(const CartTopo& topo, const SlabLayout& L);
-cudaError_t launch_heat3d_pull(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
-                               double kappa, double dt, const double inv_h2[3], cudaStream_t s);
-
-// The same step with each CTA's tile and its six halo faces staged by
-// tensor copies (TMA) onto one mbarrier; needs an even block width too.  A
-// wait for the copies that gives up sets *err (the context's device word).
-bool heat3d_tma_supported(const CartTopo& topo, const SlabLayout& L);
-cudaError_t launch_heat3d_tma(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
-                              double kappa, double dt, const double inv_h2[3], int* err, cudaStream_t s);
+// Heat in 2-D and 3-D, ghost width 1 (lg_heat.cu): `steps` (1 or 2) forward-
+// Euler steps in one launch, or one half (0: stages 1 and 2, 1: stages 3 and
+// 4) of a RungeKutta4 step.  Halos come from the neighbour blocks' interiors;
+// `out` gets interiors only (its ghost columns are scratch).  RungeKutta4:
+// half 0 reads the state from `in` and leaves y + dt/2 k2 in `out` and the
+// running sum of the axpys in `aux`; half 1 reads those from `in` and `aux`
+// and the state from `y`.  Bit-identical to the reference's steps.
+bool heat_march_supported(const CartTopo& topo, const SlabLayout& L);
+cudaError_t launch_heat_march_fe(int steps, const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
+                                 int field, const int periodic[3], double kappa, double dt, const double inv_h2[3],
+                                 cudaStream_t s);
+cudaError_t launch_heat_march_rk4(int half, const double* in, double* out, const double* y, double* aux,
+                                  const CartTopo& topo, const SlabLayout& L, int field, const int periodic[3],
+                                  double kappa, double dt, const double inv_h2[3], cudaStream_t s);
 
 // (a) fused Model C Euler-Maruyama step, FP64, bit-exact to the reference.
 // Reads phi (field 0) and u (field 1) from `in`, writes both to `out` with
