@@ -64,26 +64,22 @@ __host__ __device__ __forceinline__ double unit_open(uint64_t bits) {
 
 constexpr double kTau = 6.283185307179586476925286766559;
 
-// ln u for the Box-Muller radius, u in [2^-53, 1], within 3.5e-16 relative
-// of the exact logarithm (the Gaussian is held to 1e-12 of glibc's).  A
-// table-driven reduction (the method of Tang, ACM TOMS 16, 1990, with the
-// table holding the logarithm of its own rounded reciprocals): u = 2^e f
-// with f in [sqrt(1/2), sqrt(2)), F_j = 1 + j/128 the nearest centre
-// (j = rint((f - 1) 128), f - 1 exact), r = f RN(1/F_j) - 1 by one fma
-// (|r| <= 0.0055), and ln u = e ln 2 + L_j + log1p(r) with
-// L_j = -ln RN(1/F_j) from lg_log_table.h and log1p by its Taylor series to
-// r^7 (truncation below 2e-17 relative).  The centre F_0 = 1 makes r = f - 1
-// exact next to u = 1, where ln u is tiny; ln 2 is split so that e ln2_hi
-// is exact.  u = 1 gives exactly +0.
-__device__ __forceinline__ double log_unit_interval(double u) {
-    const long long bu = __double_as_longlong(u);
-    int e = (int)((bu >> 52) & 0x7ff) - 1023;
-    double f = __longlong_as_double((bu & 0x000fffffffffffffLL) | 0x3ff0000000000000LL);
-    if (f > 1.4142135623730951) {
-        f = 0.5 * f;
-        e += 1;
-    }
-    const int j = __double2int_rn((f - 1.0) * 128.0);
+// ln u for the Box-Muller radius, u = n 2^-53 with n = 1 .. 2^53 exact in a
+// double, within 3.5e-16 relative of the exact logarithm (the Gaussian is
+// held to 1e-12 of glibc's).  A table-driven reduction (the method of Tang,
+// ACM TOMS 16, 1990, with the table holding the logarithm of its own rounded
+// reciprocals): u = 2^e f with f in [sqrt(1/2), sqrt(2)) by the high word,
+// F_j = 1 + j/128 the nearest centre (128 f - 128 rounded to an integer by
+// one fma with 1.5 2^52), r = f RN(1/F_j) - 1 by one fma (|r| <= 0.0055), and
+// ln u = e ln 2 + L_j + log1p(r) with L_j = -ln RN(1/F_j) from lg_log_table.h
+// and log1p by its Taylor series to r^7 (truncation below 2e-17 relative).
+// The centre F_0 = 1 makes r = f - 1 exact next to u = 1, where ln u is tiny;
+// ln 2 is split so that e ln2_hi is exact.  u = 1 gives exactly +0.
+__device__ __forceinline__ double log_unit_interval(double n) {
+    const int hx = __double2hiint(n) + (0x3ff00000 - 0x3fe6a09e);
+    const int e = (hx >> 20) - (0x3ff + 53);
+    const double f = __hiloint2double((hx & 0x000fffff) + 0x3fe6a09e, __double2loint(n));
+    const int j = __double2loint(fma(f, 128.0, 0x1.8p52 - 128.0));
     const double2 E = __ldg(&kLogTable[j - kLogTableMin]);
     const double r = fma(f, E.x, -1.0);
     double q = 1.0 / 7.0;
@@ -97,55 +93,54 @@ __device__ __forceinline__ double log_unit_interval(double u) {
     return fma((double)e, ln2_hi, E.y) + fma((double)e, ln2_lo, p);
 }
 
-// cos x for the Box-Muller angle, x = fl(2 pi v) in (0, 2 pi], to about
-// 1e-15 relative also next to the zeros of cos: Cody-Waite reduction
-// r = x - k pi/2 with pi/2 in three parts (the first two of 33 bits, so
-// k C1 and k C2 are exact and the two leading subtractions cancel exactly),
-// then the sine or cosine Taylor polynomial of r (|r| <= pi/4, truncated at
-// r^15 / r^16) and the quadrant's sign.
-__device__ __forceinline__ double cos_full_turn(double x) {
-    const double t = x * 0x1.45f306dc9c883p-1;  // x 2/pi
-    const double magic = 0x1.8p52;               // t + magic rounds t to an integer (ties to even)
-    const double kq = t + magic;
-    const int q = __double2loint(kq) & 3;
-    const double kd = kq - magic;
-    double r = fma(-kd, 0x1.921fb544p+0, x);
-    r = fma(-kd, 0x1.0b4611a6p-34, r);
-    r = fma(-kd, 0x1.3198a2e037073p-69, r);
+// cos x for the Box-Muller angle, x = fl(2 pi v) in (0, 2 pi], `upper` where
+// v > 1/2, to about 2e-16 relative also next to the zeros of cos: x in the
+// lower half is pi/2 + r, in the upper half 3 pi/2 + r, |r| <= pi/2, and
+// cos x = -sin r, sin r.  The centre is subtracted in two parts (the first
+// subtraction is exact next to the zero); sin r = r + r z Q(z), z = r^2, Q
+// the polynomial of degree 7 that minimises the relative error on that
+// interval (Remez exchange; 2.8e-19).
+__device__ __forceinline__ double cos_full_turn(double x, bool upper) {
+    const double c_hi = upper ? 0x1.2d97c7f3321d2p+2 : 0x1.921fb54442d18p+0;
+    const double c_lo = upper ? 0x1.a79394c9e8a0ap-53 : 0x1.1a62633145c07p-54;
+    const double r = (x - c_hi) - c_lo;
     const double z = r * r;
-    // both polynomials, then a select (the lanes of a warp draw random
-    // quadrants, so a branch would run both anyway, in two halves)
-    double sp = 1.0 / 1307674368000.0;  // r - r^3/3! + r^5/5! - ... to r^15
-    sp = fma(sp, z, -1.0 / 6227020800.0);
-    sp = fma(sp, z, 1.0 / 39916800.0);
-    sp = fma(sp, z, -1.0 / 362880.0);
-    sp = fma(sp, z, 1.0 / 5040.0);
-    sp = fma(sp, z, -1.0 / 120.0);
-    sp = fma(sp, z, 1.0 / 6.0);
-    const double sv = fma(-(r * z), sp, r);
-    double cp = 1.0 / 20922789888000.0;  // 1 - r^2/2! + r^4/4! - ... to r^16
-    cp = fma(cp, z, -1.0 / 87178291200.0);
-    cp = fma(cp, z, 1.0 / 479001600.0);
-    cp = fma(cp, z, -1.0 / 3628800.0);
-    cp = fma(cp, z, 1.0 / 40320.0);
-    cp = fma(cp, z, -1.0 / 720.0);
-    cp = fma(cp, z, 1.0 / 24.0);
-    cp = fma(cp, z, -0.5);
-    const double cv = fma(z, cp, 1.0);
-    const double v = (q & 1) ? sv : cv;
-    return (q == 1 || q == 2) ? -v : v;
+    double q = 0x1.8829a29fbb6b6p-49;
+    q = fma(q, z, -0x1.ae431d97313e9p-41);
+    q = fma(q, z, 0x1.6123cb2907df4p-33);
+    q = fma(q, z, -0x1.ae6454cb57936p-26);
+    q = fma(q, z, 0x1.71de3a5287c8ap-19);
+    q = fma(q, z, -0x1.a01a01a0148bdp-13);
+    q = fma(q, z, 0x1.11111111110c1p-7);
+    q = fma(q, z, -0x1.5555555555555p-3);
+    const double s = fma(r * z, q, r);
+    return __hiloint2double(__double2hiint(s) ^ (upper ? 0 : 0x80000000), __double2loint(s));
+}
+
+// sqrt w for w = 0 or 2^-60 < w < 2^60, within an ulp: g = w y with y the
+// hardware's approximation of 1 / sqrt(w) (better than 2^-19), then the cubic
+// Householder step g (1 + e/2 + 3 e^2 / 8), e = 1 - g y.  A zero of either
+// sign gives itself (the approximation's infinity is made finite).
+__device__ __forceinline__ double sqrt_radius(double w) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(w));
+    y = __hiloint2double(min(__double2hiint(y) & 0x7fffffff, 0x7fe00000), 0);
+    const double g = w * y;
+    const double e = fma(-g, y, 1.0);
+    return fma(g * e, fma(e, 0.375, 0.5), g);
 }
 
 // Box-Muller cosine branch from one key (src/util/rng.rs:43-49): the
-// integer stream and the uniforms are exact; the transcendental factors
-// (log_unit_interval, cos_full_turn and the square root) are within about
-// 1e-15 of glibc's, the Gaussian within 1e-12 relative as required.
+// integer stream and the uniforms are exact (n 2^-53 with n = (bits >> 11) +
+// 1); the transcendental factors are within a few ulp of exact, the Gaussian
+// within 1e-12 relative of the reference's as required.
 __device__ __forceinline__ double standard_normal(uint64_t key) {
-    uint64_t a = splitmix64(key);
-    uint64_t b = splitmix64(a ^ 0xD1B54A32D192ED03ull);
-    double u = unit_open(a);
-    double v = unit_open(b);
-    return sqrt(-2.0 * log_unit_interval(u)) * cos_full_turn(kTau * v);
+    const uint64_t a = splitmix64(key);
+    const uint64_t b = splitmix64(a ^ 0xD1B54A32D192ED03ull);
+    const double nu = (double)((a >> 11) + 1), nv = (double)((b >> 11) + 1);
+    // fl(2 pi v): the power of two scales exactly
+    const double x = nv * (kTau * (1.0 / 9007199254740992.0));
+    return sqrt_radius(-2.0 * log_unit_interval(nu)) * cos_full_turn(x, (int64_t)b < 0);
 }
 
 // Single-precision Gaussian from the same two uniforms, for the FP32 path.
