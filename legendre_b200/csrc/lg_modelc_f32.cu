@@ -20,6 +20,7 @@ struct Fast32 {
     float lambda, d_thermal, inv_h2_flux, ih0, ih1;
     float f_a_bar, f_a1pe, f_2ae, f_a12, f_tol;  // flux: a, a(1+e'), 2 a e', a12, tol
     float c_a_bar, c_a1pe, c_2ae, c_tol;         // cell-centred anisotropy
+    int far_key;
 };
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -106,22 +107,13 @@ struct OpsFast32 {
     // reciprocal the general form takes.  Same values as the general forms
     // with the flat selects taken.
     static __device__ __forceinline__ float quarter(float d1, float c, float e) { return 0.25f * ((d1 + c) - e); }
-    static __device__ __forceinline__ float face_mag2(float dx, float dy) {
-        const float s = dx * dx + dy * dy;
-        return s * s;
+    static __device__ __forceinline__ int far_key(const Fast32& m) { return m.far_key; }
+    static __device__ __forceinline__ int face_key(float dx, float dy) { return order_key(dx * dx + dy * dy); }
+    static __device__ __forceinline__ int center_key(float cdx, float cdy) {
+        return quarter_key(cdx * cdx + cdy * cdy);
     }
-    static __device__ __forceinline__ bool face_flat(const Fast32& m, float dx, float dy) {
-        return face_mag2(dx, dy) <= m.f_tol;
-    }
-    static __device__ __forceinline__ bool center_flat(const Fast32& m, float cdx, float cdy) {
-        return face_mag2(0.5f * cdx, 0.5f * cdy) <= m.c_tol;
-    }
-    static __device__ __forceinline__ float xface_far(const Fast32& m, float dn, float) {
-        return m.f_a_bar * (m.f_a_bar * dn);
-    }
-    static __device__ __forceinline__ float yface_far(const Fast32& m, float dn, float) {
-        return m.f_a_bar * (m.f_a_bar * dn);
-    }
+    static __device__ __forceinline__ float xface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
+    static __device__ __forceinline__ float yface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ void cell_far(const Fast32& m, float jr, float jl, float jt, float jb, float p,
                                                     float uc, float ul, float ur, float up, float um, float& kphi,
                                                     float& ku) {
@@ -171,6 +163,7 @@ Fast32 fast32_of(const ModelCDev& m) {
     f.c_a1pe = (float)(m.a_bar * (1.0 + m.eps_prime));
     f.c_2ae = (float)(2.0 * m.a_bar * m.eps_prime);
     f.c_tol = (float)m.tol;
+    f.far_key = far_key_of(std::min(f.f_tol, f.c_tol));
     return f;
 }
 }  // namespace

@@ -3,6 +3,10 @@
 // with -fmad=false (see lg_kernels.cu).
 #pragma once
 
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
 #include "lg_common.cuh"
 #include "lg_kernels.h"
 
@@ -12,7 +16,42 @@ template <class T>
 struct MC {
     T lambda, d_thermal, a_bar, eps_prime, tol, f_a_bar, f_eps_prime, f_a12, f_tol, inv_h2_flux, ih0, ih1;
     T c_far, inv_c_far;  // a_bar * a_bar, the far-field mobility divisor, and RN(1 / c_far)
+    int far_key;         // largest gradient key that is flat for certain (see gradient_key)
 };
+
+// The high half of a non-negative double, or the bits of a non-negative
+// float, ordered as the values are.
+__host__ __device__ __forceinline__ int order_key(double s) {
+#ifdef __CUDA_ARCH__
+    return __double2hiint(s);
+#else
+    int64_t b;
+    memcpy(&b, &s, sizeof b);
+    return (int)(b >> 32);
+#endif
+}
+__host__ __device__ __forceinline__ int order_key(float s) {
+#ifdef __CUDA_ARCH__
+    return __float_as_int(s);
+#else
+    int b;
+    memcpy(&b, &s, sizeof b);
+    return b;
+#endif
+}
+// a key of s / 4
+__device__ __forceinline__ int quarter_key(double s) { return order_key(s) - (2 << 20); }
+__device__ __forceinline__ int quarter_key(float s) { return order_key(s) - (2 << 23); }
+
+// The far field (|grad|^4 <= tol, in the reference's rounding) decided
+// without its rounding: every |grad|^2 whose key is at most far_key_of(tol)
+// is below sqrt(tol) by more than any rounding of the sum and its square.
+template <class T>
+inline int far_key_of(T tol) {
+    if (!(tol > T(0))) return -0x7fffffff - 1;
+    const T s = std::sqrt(tol) * (T(1) - (sizeof(T) == 8 ? T(0x1p-40) : T(0x1p-20)));
+    return order_key(s) - 1;
+}
 
 template <class T>
 inline MC<T> to_mc(const ModelCDev& m) {
@@ -31,10 +70,61 @@ inline MC<T> to_mc(const ModelCDev& m) {
     r.ih1 = (T)m.inv_h2[1];
     r.c_far = r.a_bar * r.a_bar;
     r.inv_c_far = T(1) / r.c_far;
+    r.far_key = far_key_of(std::min(r.f_tol, r.tol));
     return r;
 }
 
-// KarmaRappelFlux::face (finite_volume.rs:129-142)
+// RN(1 / c) for 2^-900 <= |c| <= 2^900: the hardware's approximation (better
+// than 2^-19), one cubic step, y (1 + e + e^2) with e = 1 - c y, and one
+// correction with the exact residual, which gives the correctly rounded
+// reciprocal unless every bit of c's mantissa is set (Markstein, IBM J. Res.
+// Dev. 34, 1990).
+__device__ __forceinline__ double recip_rn(double c) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(c));
+    double e = fma(-c, y, 1.0);
+    e = fma(e, e, e);
+    y = fma(y, e, y);
+    return fma(y, fma(-c, y, 1.0), y);
+}
+// RN(x / c) with y = RN(1 / c): the quotient RN(x y) corrected with its exact
+// residual (the same theorem).  Against the division on 1.2e9 operands, near
+// rounding midpoints and with mantissas of all ones among them: no mismatch.
+// x = 0 gives a zero (its sign is not kept).
+__device__ __forceinline__ double quotient_rn(double x, double c, double y) {
+    const double q = x * y;
+    return fma(fma(-q, c, x), y, q);
+}
+// 2^-900 <= |c| < 2^900, where recip_rn holds
+__device__ __forceinline__ bool recip_range(double c) {
+    return (unsigned)(__double2hiint(c) & 0x7fffffff) - 0x07b00000u < 0x70800000u;
+}
+
+// the division itself, out of line: for operands outside the ranges above
+static __device__ __noinline__ double ieee_quotient(double x, double c) { return x / c; }
+
+// the two ratios of a non-flat face: n1 / c and n2 / c, the IEEE quotients
+__device__ __forceinline__ void ratios(double n1, double n2, double c, double& q1, double& q2) {
+    if (recip_range(c)) {
+        const double y = recip_rn(c);
+        q1 = quotient_rn(n1, c, y);
+        q2 = quotient_rn(n2, c, y);
+    } else {
+        q1 = ieee_quotient(n1, c);
+        q2 = ieee_quotient(n2, c);
+    }
+}
+__device__ __forceinline__ void ratios(float n1, float n2, float c, float& q1, float& q2) {
+    q1 = n1 / c;
+    q2 = n2 / c;
+}
+__device__ __forceinline__ double ratio(double n, double c) {
+    return recip_range(c) ? quotient_rn(n, c, recip_rn(c)) : ieee_quotient(n, c);
+}
+__device__ __forceinline__ float ratio(float n, float c) { return n / c; }
+
+// KarmaRappelFlux::face (finite_volume.rs:129-142); its two quotients share
+// one reciprocal
 template <class T>
 __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da) {
     T dx2 = dx * dx;
@@ -45,8 +135,10 @@ __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da)
         a = m.f_a_bar;
         da = T(0);
     } else {
-        a = m.f_a_bar * (T(1) + m.f_eps_prime * (dx2 * dx2 + dy2 * dy2) / mag2);
-        da = -(m.f_a12) * dx * dy * (dx2 - dy2) / mag2;
+        T q1, q2;
+        ratios(m.f_eps_prime * (dx2 * dx2 + dy2 * dy2), -(m.f_a12) * dx * dy * (dx2 - dy2), mag2, q1, q2);
+        a = m.f_a_bar * (T(1) + q1);
+        da = q2;
     }
 }
 
@@ -59,7 +151,7 @@ __device__ __forceinline__ T center_anisotropy(const MC<T>& m, T dx, T dy) {
     T sum = dx2 + dy2;
     T mag2 = sum * sum;
     if (mag2 <= m.tol) return m.a_bar;
-    return m.a_bar * (T(1) + m.eps_prime * (dx2 * dx2 + dy2 * dy2) / mag2);
+    return m.a_bar * (T(1) + ratio(m.eps_prime * (dx2 * dx2 + dy2 * dy2), mag2));
 }
 
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
@@ -76,13 +168,21 @@ __device__ __forceinline__ double normal_t(uint64_t key, double) { return standa
 // 600 divisors, half of them next to rounding midpoints).  Zeros are x y
 // (their sign kept); tiny and huge x take the division.
 __device__ __forceinline__ double div_far(double x, double c, double y) {
-    const double ax = fabs(x);
     const double q = x * y;
     const double qc = fma(fma(-q, c, x), y, q);
-    if (ax >= 0x1p-960 && ax <= 0x1p+960) return qc;
-    return x == 0.0 ? q : x / c;  // +-0 / c = +-0 = +-0 y (y > 0)
+    const unsigned ex = (unsigned)__double2hiint(x) << 1;  // exponent above the sign
+    const bool in = ex - 0x07e00000u < 0xf0200000u;  // 2^-960 <= |x| < 2^961
+    if (!in && x != 0.0) return ieee_quotient(x, c);
+    return in ? qc : q;  // +-0 / c = +-0 = +-0 y (y > 0)
 }
 __device__ __forceinline__ float div_far(float x, float c, float) { return x / c; }
+// x / c, the IEEE quotient, for the mobility divisor c = a^2 of one cell
+__device__ __forceinline__ double div_cell(double x, double c) {
+    const unsigned ex = (unsigned)__double2hiint(x) << 1;  // exponent above the sign
+    if (ex - 0x0f600000u < 0xe1000000u && recip_range(c)) return quotient_rn(x, c, recip_rn(c));
+    return ieee_quotient(x, c);
+}
+__device__ __forceinline__ float div_cell(float x, float c) { return x / c; }
 __device__ __forceinline__ float normal_t(uint64_t key, float) { return standard_normal_f32(key); }
 
 // The exact FP64 arithmetic policy of the step kernels: face fluxes from
@@ -110,30 +210,18 @@ struct OpsExact {
         return a * (a * dn + da * dt);
     }
     // The far-field forms: the face fluxes and the cell update with the
-    // anisotropy branches decided (kr_face and center_anisotropy both flat),
-    // the same expressions as the branches they stand for, so their bits.
-    // `quarter` is the transverse quarter sum of xface / yface and the
-    // *_mag2 the |grad|^4 those branches test.
+    // anisotropy branches decided (kr_face and center_anisotropy both flat):
+    // a = f_a_bar, da = 0, and a dn - 0 dt is a dn (the transverse difference
+    // is finite where the test holds).  The test is conservative (far_key_of):
+    // a pass that fails it takes the general path, whose branches decide each
+    // face in the reference's rounding.
     static __device__ __forceinline__ T quarter(T d1, T c, T e) { return T(0.25) * (d1 + c - e); }
-    static __device__ __forceinline__ T face_mag2(T dx, T dy) {
-        const T dx2 = dx * dx;
-        const T dy2 = dy * dy;
-        const T sum = dx2 + dy2;
-        return sum * sum;
-    }
-    static __device__ __forceinline__ T center_mag2(T cdx, T cdy) { return face_mag2(T(0.5) * cdx, T(0.5) * cdy); }
-    static __device__ __forceinline__ bool face_flat(const MC<T>& m, T dx, T dy) { return face_mag2(dx, dy) <= m.f_tol; }
-    static __device__ __forceinline__ bool center_flat(const MC<T>& m, T cdx, T cdy) {
-        return center_mag2(cdx, cdy) <= m.tol;
-    }
-    static __device__ __forceinline__ T xface_far(const MC<T>& m, T dn, T dt) {
-        const T a = m.f_a_bar, da = T(0);
-        return a * (a * dn - da * dt);
-    }
-    static __device__ __forceinline__ T yface_far(const MC<T>& m, T dn, T dt) {
-        const T a = m.f_a_bar, da = T(0);
-        return a * (a * dn + da * dt);
-    }
+    static __device__ __forceinline__ int far_key(const MC<T>& m) { return m.far_key; }
+    static __device__ __forceinline__ int face_key(T dx, T dy) { return order_key(fma_t(dx, dx, dy * dy)); }
+    // from the whole differences p(i+1) - p(i-1)
+    static __device__ __forceinline__ int center_key(T cdx, T cdy) { return quarter_key(fma_t(cdx, cdx, cdy * cdy)); }
+    static __device__ __forceinline__ T xface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
+    static __device__ __forceinline__ T yface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ void cell_far(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T uc, T ul, T ur,
                                                     T up, T um, T& kphi, T& ku) {
         const T flux = (jr - jl + jt - jb) * m.inv_h2_flux;
@@ -156,7 +244,7 @@ struct OpsExact {
         const T num = fma_t(m.lambda * uc, -p_prime, flux - g_prime);
         // a == a_bar: the divisor a a is c_far (whichever branch of the
         // anisotropy gave it)
-        kphi = a == m.a_bar ? div_far(num, m.c_far, m.inv_c_far) : num / (a * a);
+        kphi = a == m.a_bar ? div_far(num, m.c_far, m.inv_c_far) : div_cell(num, a * a);
         T acc = T(0);
         acc += ((ur - (uc + uc)) + ul) * m.ih0;
         acc += ((up - (uc + uc)) + um) * m.ih1;
@@ -187,7 +275,8 @@ struct OpsExact {
         const T dx = T(0.5) * cdx, dy = T(0.5) * cdy;
         T a, da;
         kr_face(m, c0 * dx + s0 * dy, c0 * dy - s0 * dx, a, da);
-        kphi = fma_t(m.lambda * uc, -p_prime, flux - g_prime) / (a * a);
+        const T num = fma_t(m.lambda * uc, -p_prime, flux - g_prime);
+        kphi = a == m.f_a_bar ? div_far(num, m.c_far, m.inv_c_far) : div_cell(num, a * a);
         T acc = T(0);
         acc += ((ur - (uc + uc)) + ul) * m.ih0;
         acc += ((up - (uc + uc)) + um) * m.ih1;

@@ -565,24 +565,22 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             T kphi0, ku0, kphi1, ku1;
             bool far = false;
             if constexpr (Ops::kFarPass) {
-                // the four faces' and two centres' anisotropy tests; where
-                // they are all flat across the warp (the far field) the pass
-                // runs without branches, the same expressions as the general
-                // path
+                // the four faces' and two centres' gradients; where all are
+                // flat for certain across the warp (the far field) the pass
+                // runs without branches, with the general path's values
                 const T xn0 = B.b - B.a, xt0 = Ops::quarter(C.b - A.b, C.a, A.a);
                 const T yn0 = C.b - B.b, yt0 = Ops::quarter(C.c - C.a, B.c, B.a);
                 const T xn1 = C.b - C.a, xt1 = Ops::quarter(D.b - B.b, D.a, B.a);
                 const T yn1 = D.b - C.b, yt1 = Ops::quarter(D.c - D.a, C.c, C.a);
-                const bool flat = Ops::face_flat(m, xn0, xt0) && Ops::face_flat(m, yt0, yn0) &&
-                                  Ops::face_flat(m, xn1, xt1) && Ops::face_flat(m, yt1, yn1) &&
-                                  Ops::center_flat(m, B.c - B.a, C.b - A.b) &&
-                                  Ops::center_flat(m, C.c - C.a, D.b - B.b);
-                far = __all_sync(kFull, flat);
+                const int key = max(max(max(Ops::face_key(xn0, xt0), Ops::face_key(yt0, yn0)),
+                                        max(Ops::face_key(xn1, xt1), Ops::face_key(yt1, yn1))),
+                                    max(Ops::center_key(B.c - B.a, C.b - A.b), Ops::center_key(C.c - C.a, D.b - B.b)));
+                far = __all_sync(kFull, key <= Ops::far_key(m));
                 if (far) {
-                    fl0 = Ops::xface_far(m, xn0, xt0);
-                    jt0 = Ops::yface_far(m, yn0, yt0);
-                    fl1 = Ops::xface_far(m, xn1, xt1);
-                    jt1 = Ops::yface_far(m, yn1, yt1);
+                    fl0 = Ops::xface_far(m, xn0);
+                    jt0 = Ops::yface_far(m, yn0);
+                    fl1 = Ops::xface_far(m, xn1);
+                    jt1 = Ops::yface_far(m, yn1);
                     T fr0 = __shfl_down_sync(kFull, fl0, 1), fr1 = __shfl_down_sync(kFull, fl1, 1);
                     if (lane == last_lane) {
                         fr0 = fb0;
@@ -654,9 +652,11 @@ __global__ void __launch_bounds__(256, MINB)
 
     const int64_t first_listed = (int64_t)gridDim.x * wpc;
     for (int64_t unit = (int64_t)blockIdx.x * wpc + (threadIdx.x >> 5); unit < g.units;) {
-        const int s = (int)(unit % g.strips);
-        const int k = (int)((unit / g.strips) % g.chunks);
-        const int b = (int)(unit / ((int64_t)g.strips * g.chunks));
+        // 32-bit divisions: a grid holds fewer than 2^32 units
+        const unsigned bk = (unsigned)unit / (unsigned)g.strips;
+        const int s = (int)((unsigned)unit - bk * (unsigned)g.strips);
+        const int b = (int)(bk / (unsigned)g.chunks);
+        const int k = (int)(bk - (unsigned)b * (unsigned)g.chunks);
         // units are g.rows high (a multiple of NB unless TAIL); a block's
         // last unit ends on its last row and may overlap the one before it,
         // whose rows it then recomputes to the same bits
