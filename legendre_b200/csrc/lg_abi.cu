@@ -596,14 +596,14 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
              p->d_thermal, p->noise_amplitude, p->anisotropy_tol, p->flux_tol, dt, (unsigned long long)seed, variant,
              st->orient);
     const int64_t ncells = st->grid->nblocks * st->grid->block[0] * st->grid->block[1];
-    // variant = kind + 1000 * rows: kind 0 library default, 1 one thread per
-    // cell in reference order, 2/3/4 warp strips with 2/3/4 CTAs per SM, 5/6/7
+    // variant = kind + 1000 * rows: kind 0 library default (paired rows on the
+    // work list, 2 CTAs per SM), 1 one thread per cell in reference order, 2/3/4 warp strips with 2/3/4 CTAs per SM, 5/6/7
     // the same with two rows per pass of the row loop, 12..17 those forms as
     // a persistent work list; rows fixes the strip height
     const int kind = variant % 1000 % 10, rows = variant / 1000;
-    const bool listed = variant % 1000 >= 10;
+    const bool listed = kind == 0 || variant % 1000 >= 10;
     const bool tile = kind != 1 && lg::modelc_tile_supported(topo);
-    const int minb = kind >= 2 ? kind : (st->dtype == LG_F32 ? 3 : 2);
+    const int minb = kind >= 2 ? kind : 5;
     unsigned* work = listed ? reinterpret_cast<unsigned*>(st->d_t + 2) : nullptr;
     // the run's first step takes its units from a cleared list (each step
     // clears the other slot's list for the step after it)
@@ -617,10 +617,10 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
             e = st->dtype == LG_F64
                     ? lg::launch_modelc_oriented_f64(static_cast<const double*>(in), static_cast<double*>(out), topo,
                                                      L, m, dt, nz, st->d_t, st->tslot,
-                                                     static_cast<const double*>(st->orient), ncells, rows, ctx->stream)
+                                                     static_cast<const double*>(st->orient), ncells, rows, work, ctx->stream)
                     : lg::launch_modelc_oriented_f32(static_cast<const float*>(in), static_cast<float*>(out), topo, L,
                                                      m, dt, nz, st->d_t, st->tslot,
-                                                     static_cast<const float*>(st->orient), ncells, rows, ctx->stream);
+                                                     static_cast<const float*>(st->orient), ncells, rows, work, ctx->stream);
         else if (st->dtype == LG_F64)
             e = tile ? lg::launch_modelc_tile_f64(static_cast<const double*>(in), static_cast<double*>(out), topo, L,
                                                   m, dt, nz, st->d_t, st->tslot, rows, minb, work, ctx->stream)

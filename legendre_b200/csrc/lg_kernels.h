@@ -96,10 +96,10 @@ cudaError_t launch_modelc_tile_f32(const float* in, float* out, const CartTopo& 
 // the reference's apply_oriented path.
 cudaError_t launch_modelc_oriented_f64(const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                        const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
-                                       const double* trig, int64_t ncells, int rows, cudaStream_t s);
+                                       const double* trig, int64_t ncells, int rows, unsigned* work, cudaStream_t s);
 cudaError_t launch_modelc_oriented_f32(const float* in, float* out, const CartTopo& topo, const SlabLayout& L,
                                        const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
-                                       const float* trig, int64_t ncells, int rows, cudaStream_t s);
+                                       const float* trig, int64_t ncells, int rows, unsigned* work, cudaStream_t s);
 
 // One RungeKutta4 stage of Model C without noise (rk4.rs:40-79) on the
 // strip schedule: mode 1 writes the drift of `in` to k and y + c k to out;

@@ -24,8 +24,8 @@ cudaError_t launch_modelc_tile_f64(const double* in, double* out, const CartTopo
 
 cudaError_t launch_modelc_oriented_f64(const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                        const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
-                                       const double* trig, int64_t ncells, int rows, cudaStream_t s) {
-    TileArgs g{topo, L, dt, nz.seed, tdev, slot, rows, 0, 0, 0};
+                                       const double* trig, int64_t ncells, int rows, unsigned* work, cudaStream_t s) {
+    TileArgs g{topo, L, dt, nz.seed, tdev, slot, rows, 0, 0, 0, work};
     const MC<double> mc = to_mc<double>(m);
     const double scale_amp = std::sqrt(dt) * nz.amp;
     const OrientArgs oa{trig, ncells};

@@ -180,8 +180,8 @@ cudaError_t launch_modelc_tile_f32(const float* in, float* out, const CartTopo& 
 
 cudaError_t launch_modelc_oriented_f32(const float* in, float* out, const CartTopo& topo, const SlabLayout& L,
                                        const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
-                                       const float* trig, int64_t ncells, int rows, cudaStream_t s) {
-    TileArgs g{topo, L, dt, nz.seed, tdev, slot, rows, 0, 0, 0};
+                                       const float* trig, int64_t ncells, int rows, unsigned* work, cudaStream_t s) {
+    TileArgs g{topo, L, dt, nz.seed, tdev, slot, rows, 0, 0, 0, work};
     const Fast32 f = fast32_of(m);
     const float scale_amp = (float)(std::sqrt(dt) * nz.amp);
     const OrientArgs oa{trig, ncells};

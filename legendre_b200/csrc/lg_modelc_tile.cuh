@@ -222,9 +222,9 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
     const int sy = NX > 0 ? NX + 2 : g.L.gdim[0];
     // lanes past the block's last column (valid false) run the same code on
     // a clamped column and only skip the stores: no branch splits the face,
-    // noise and cell arithmetic.  Unit heights are whole groups of NB rows,
-    // so the row loop has no separately unrolled tail; only blocks of fewer
-    // than NB rows (TAIL) run rows past the unit's end, without stores.
+    // noise and cell arithmetic.  Unit heights are whole groups of rows
+    // (strip_group), so an unrolled row loop has no separate tail; only blocks
+    // of fewer rows (TAIL) run rows past the unit's end, without stores.
     // rows below rs belong to the unit below (a block's last unit overlaps
     // it): computed for their faces, stored only by their own unit
     const bool live = (!TAIL || j < r1) && j >= rs;
@@ -412,8 +412,8 @@ __device__ __forceinline__ void strip_unit(const typename Ops::Params& m, uint64
 // reads its four phi and u rows j-1 .. j+2 from L1, where the previous pass
 // prefetched them, instead of carrying a six-row window in registers: the
 // unit needs fewer registers (no spills at 3 CTAs per SM) and no register
-// moves to shift the window.  Units are a multiple of four rows ending at
-// or before the ghost row n1, so every row read lies inside the slab.
+// moves to shift the window.  Units are an even number of rows ending at or
+// before the ghost row n1, so every row read lies inside the slab.
 // Same arithmetic per cell, in the same operand order, as strip_row.
 //
 // ORIENT: the multi-grain faces (strip_row's ORIENT branch, for two rows):
@@ -625,6 +625,18 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
     if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
 }
 
+// strip, row chunk and block of a work unit
+struct StripUnit {
+    int s, k, b;
+    // 32-bit divisions: a grid holds fewer than 2^32 units
+    __device__ __forceinline__ void decode(const TileArgs& g, int64_t unit) {
+        const unsigned bk = (unsigned)unit / (unsigned)g.strips;
+        s = (int)((unsigned)unit - bk * (unsigned)g.strips);
+        b = (int)(bk / (unsigned)g.chunks);
+        k = (int)(bk - (unsigned)b * (unsigned)g.chunks);
+    }
+};
+
 // Rows per work unit are at most 32, so one batch of boundary faces (lanes
 // across rows) serves the whole unit.
 template <class T, class Ops, bool NOISE, int MINB, int NX, int PF, bool BATCH = false, bool TAIL = false,
@@ -640,6 +652,21 @@ __global__ void __launch_bounds__(256, MINB)
     const int lane = threadIdx.x & 31;
     const int wpc = blockDim.x >> 5;
 
+    const int64_t first_listed = (int64_t)gridDim.x * wpc;
+    int64_t unit = (int64_t)blockIdx.x * wpc + (threadIdx.x >> 5);
+    // what does not depend on the previous step: the first unit's place and
+    // its neighbours in the topology
+    StripUnit su;
+    Nbr2 nb{};
+    if (unit < g.units) {
+        su.decode(g, unit);
+        nb.load(topo, su.b);
+    }
+    // programmatic dependent launch: wait for the previous step's writes,
+    // then let the next step's CTAs become resident
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
     // Simulation::t lives on the device in two slots: this step reads
     // tdev[slot] (its bits are the Wiener salt, euler_maruyama.rs:73) and
     // writes t + dt to the other slot (simulation.rs:285), so a captured
@@ -650,14 +677,9 @@ __global__ void __launch_bounds__(256, MINB)
         if (g.work) g.work[g.slot ^ 1] = 0u;
     }
 
-    const int64_t first_listed = (int64_t)gridDim.x * wpc;
-    for (int64_t unit = (int64_t)blockIdx.x * wpc + (threadIdx.x >> 5); unit < g.units;) {
-        // 32-bit divisions: a grid holds fewer than 2^32 units
-        const unsigned bk = (unsigned)unit / (unsigned)g.strips;
-        const int s = (int)((unsigned)unit - bk * (unsigned)g.strips);
-        const int b = (int)(bk / (unsigned)g.chunks);
-        const int k = (int)(bk - (unsigned)b * (unsigned)g.chunks);
-        // units are g.rows high (a multiple of NB unless TAIL); a block's
+    while (unit < g.units) {
+        const int s = su.s, k = su.k, b = su.b;
+        // units are g.rows high (whole groups of rows unless TAIL); a block's
         // last unit ends on its last row and may overlap the one before it,
         // whose rows it then recomputes to the same bits
         int r0 = k * g.rows;
@@ -678,8 +700,6 @@ __global__ void __launch_bounds__(256, MINB)
         const T* uu = in + slab_base(g.L, b, 1);
         T* po = out + slab_base(g.L, b, 0);
         T* uo = out + slab_base(g.L, b, 1);
-        Nbr2 nb;
-        nb.load(topo, b);
         if constexpr (PAIR) {
             static_assert(MODE == 0 && !TAIL && !(ORIENT && BATCH), "the paired rows serve the Euler-Maruyama step");
             if constexpr (BATCH) {
@@ -715,41 +735,87 @@ __global__ void __launch_bounds__(256, MINB)
         } else {
             unit += first_listed;
         }
+        if (unit < g.units) {
+            su.decode(g, unit);
+            nb.load(topo, su.b);
+        }
     }
 }
 
-// Rows per work unit: at most 32 (one batch of boundary faces per unit),
-// fewer only when the grid would otherwise hold too few warps, and a whole
-// number of groups of nb rows (the row loop's unroll) when the block has at
-// least nb rows.
-inline int strip_rows(const CartTopo& topo, int strips, int rows, int nb) {
+// Rows a unit's height is a multiple of: the paired rows step two at a time,
+// the unrolled loop (FP32 multi-grain single rows) four.
+template <class T, bool ORIENT, bool PAIR>
+constexpr int strip_group() {
+    return PAIR ? 2 : (sizeof(T) == 4 && ORIENT ? 4 : 1);
+}
+
+// Rows per work unit, where the caller leaves them open: the power of two up
+// to 32 (one batch of boundary faces per unit) that minimises the step's
+// length.  A warp spends about two rows' time on starting a unit, and a row's
+// time hardly depends on how many warps share the SM until the resident warps
+// (`slots`) are all busy; from there on the units queue (FP32 rows are short
+// enough to feel the queue from about three quarters on).  FP64 paired rows
+// at 2, 4, 8, 16 rows a unit: 64^2 4.8, 6.8, 11.0, 19.4 us a step; 512^2 8.6,
+// 8.4, 11.2, 19.5; 1008^2 25.0, 21.2, 19.8, 25.1; 2048^2 98, 77, 67, 63.
+template <class T>
+inline int strip_auto_rows(const CartTopo& topo, int strips, int64_t slots) {
     const int n1 = topo.n[1];
-    if (rows <= 0) {
-        const int64_t want_units = (int64_t)device_sm_count() * 48 * 2;
-        const int64_t per_chunk = (int64_t)topo.nblocks * strips;
-        const int chunks =
-            (int)std::max<int64_t>(1, std::min<int64_t>(n1, (want_units + per_chunk - 1) / per_chunk));
-        rows = std::max(8, (n1 + chunks - 1) / chunks);
+    const double queue = sizeof(T) == 8 ? 1.0 : 1.36;
+    int best = 2;
+    double best_cost = 0.0;
+    for (int rows = 32; rows >= 2; rows /= 2) {
+        const int h = std::min(rows, n1);
+        const double units = (double)topo.nblocks * strips * ((n1 + h - 1) / h);
+        const double cost = (h + 2) * std::max(1.0, queue * units / (double)slots);
+        if (best_cost == 0.0 || cost < best_cost) {
+            best_cost = cost;
+            best = h;
+        }
     }
-    rows = std::max(1, std::min(std::min(rows, 32), n1));
-    if (n1 >= nb) rows = std::max(nb, rows / nb * nb);
-    return rows;
+    return best;
 }
 
-// work decomposition of a launch: units of (block, strip, row chunk); true
-// when the block is lower than the row group (the TAIL kernels)
-inline bool strip_plan(TileArgs& g, int nb) {
+// work decomposition of a launch: units of (block, strip, row chunk) of
+// g.rows rows (at most 32; 0: chosen as above), a whole number of groups of
+// nb rows; true when the block is lower than the row group (the TAIL kernels)
+template <class T>
+inline bool strip_plan(TileArgs& g, int nb, int ctas_per_sm) {
     const int n0 = g.topo.n[0], n1 = g.topo.n[1];
     g.strips = (n0 + 31) / 32;
-    g.rows = strip_rows(g.topo, g.strips, g.rows, nb);
+    const int64_t slots = (int64_t)device_sm_count() * ctas_per_sm * 8;
+    int rows = g.rows > 0 ? g.rows : strip_auto_rows<T>(g.topo, g.strips, slots);
+    rows = std::max(1, std::min(std::min(rows, 32), n1));
+    if (n1 >= nb) rows = std::max(nb, rows / nb * nb);
+    g.rows = rows;
     g.chunks = (n1 + g.rows - 1) / g.rows;
     g.units = (int64_t)g.topo.nblocks * g.strips * g.chunks;
+    // one wave or less needs no list (64^2: 4.8 against 5.1 us a step)
+    if (g.units <= slots) g.work = nullptr;
     return n1 < nb;
 }
 
-inline dim3 strip_ctas(const TileArgs& g) {
+// launch with programmatic dependent launch: consecutive steps overlap one
+// step's tail with the next one's start-up (the kernel waits before it
+// touches the state)
+template <class... P, class... A>
+cudaError_t strip_launch(void (*kernel)(P...), dim3 grid, cudaStream_t s, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// CTAs of eight warps: one per eight units, or with a work list one wave
+inline dim3 strip_ctas(const TileArgs& g, int ctas_per_sm) {
     const int wpc = 8;
-    return dim3((unsigned)std::min<int64_t>((g.units + wpc - 1) / wpc, (int64_t)1 << 30));
+    const int64_t wave = g.work ? (int64_t)device_sm_count() * ctas_per_sm : (int64_t)1 << 30;
+    return dim3((unsigned)std::min<int64_t>((g.units + wpc - 1) / wpc, wave));
 }
 
 // batched instances: block widths 64 (the ensemble configuration) and 32
@@ -757,45 +823,38 @@ inline dim3 strip_ctas(const TileArgs& g) {
 // PAIR: the paired rows (256 instances of 256^2, FP32: 102.5 against 79.8 Gcell/s)
 template <class T, class Ops, bool NOISE, int MINB, bool PAIR = false>
 cudaError_t launch_strip_batch(const T* in, T* out, TileArgs g, BatchArgs bt, T dt, T scale_amp, cudaStream_t s) {
-    const bool tail = strip_plan(g, 1 + 3);
-    const dim3 grid = strip_ctas(g), block(256);
+    const bool tail = strip_plan<T>(g, strip_group<T, false, PAIR>(), MINB);
+    const dim3 grid = strip_ctas(g, MINB);
     const typename Ops::Params m{};
     if (tail) {
-        modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, true, true><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
-        return cudaGetLastError();
+        return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, true, true>, grid, s, in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
     }
     switch (g.topo.n[0]) {
-        case 32: modelc_strip_kernel<T, Ops, NOISE, MINB, 32, 1, true, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{}); break;
-        case 64: modelc_strip_kernel<T, Ops, NOISE, MINB, 64, 1, true, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{}); break;
-        default: modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, true, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
+        case 32: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 32, 1, true, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
+        case 64: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 64, 1, true, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
+        default: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, true, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, bt, OrientArgs{}, RkArgs<T>{});
     }
-    return cudaGetLastError();
 }
 
 template <class T, class Ops, bool NOISE, int MINB, int PF, bool PAIR = false>
 cudaError_t launch_strip_minb(const T* in, T* out, TileArgs g, const typename Ops::Params& m, T dt, T scale_amp,
                               cudaStream_t s) {
-    const bool tail = strip_plan(g, PF + 3);
-    dim3 grid = strip_ctas(g);
-    const dim3 block(256);
-    if (g.work)  // the work list: one wave, MINB CTAs per SM
-        grid.x = (unsigned)std::min<int64_t>(grid.x, (int64_t)device_sm_count() * MINB);
+    const bool tail = strip_plan<T>(g, strip_group<T, false, PAIR>(), MINB);
+    const dim3 grid = strip_ctas(g, MINB);
     if (tail) {  // blocks lower than the row group: single rows (the paired form needs whole groups)
-        modelc_strip_kernel<T, Ops, NOISE, MINB, 0, PF, false, true><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, BatchArgs{}, OrientArgs{}, RkArgs<T>{});
-        return cudaGetLastError();
+        return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, PF, false, true>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, OrientArgs{}, RkArgs<T>{});
     }
     const BatchArgs nob{};
     const OrientArgs noo{};
     const RkArgs<T> nork{};
     switch (g.topo.n[0]) {  // block widths of the shipped configurations get a compile-time row stride
-        case 32: modelc_strip_kernel<T, Ops, NOISE, MINB, 32, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork); break;
-        case 64: modelc_strip_kernel<T, Ops, NOISE, MINB, 64, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork); break;
-        case 126: modelc_strip_kernel<T, Ops, NOISE, MINB, 126, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork); break;
-        case 128: modelc_strip_kernel<T, Ops, NOISE, MINB, 128, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork); break;
-        case 256: modelc_strip_kernel<T, Ops, NOISE, MINB, 256, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork); break;
-        default: modelc_strip_kernel<T, Ops, NOISE, MINB, 0, PF, false, false, false, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, nob, noo, nork);
+        case 32: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 32, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
+        case 64: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 64, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
+        case 126: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 126, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
+        case 128: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 128, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
+        case 256: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 256, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
+        default: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, PF, false, false, false, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, nob, noo, nork);
     }
-    return cudaGetLastError();
 }
 
 // the multi-grain step: block widths 126 (the 101.6M-cell configuration)
@@ -805,18 +864,16 @@ cudaError_t launch_strip_minb(const T* in, T* out, TileArgs g, const typename Op
 template <class T, class Ops, bool NOISE, int MINB, bool PAIR = false>
 cudaError_t launch_strip_oriented(const T* in, T* out, TileArgs g, const typename Ops::Params& m, T dt, T scale_amp,
                                   OrientArgs oa, cudaStream_t s) {
-    const bool tail = strip_plan(g, 1 + 3);
-    const dim3 grid = strip_ctas(g), block(256);
+    const bool tail = strip_plan<T>(g, strip_group<T, true, PAIR>(), MINB);
+    const dim3 grid = strip_ctas(g, MINB);
     if (tail) {  // blocks lower than the row group: single rows
-        modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, false, true, true><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
-        return cudaGetLastError();
+        return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, false, true, true>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
     }
     switch (g.topo.n[0]) {
-        case 126: modelc_strip_kernel<T, Ops, NOISE, MINB, 126, 1, false, false, true, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{}); break;
-        case 256: modelc_strip_kernel<T, Ops, NOISE, MINB, 256, 1, false, false, true, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{}); break;
-        default: modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, false, false, true, 0, PAIR><<<grid, block, 0, s>>>(in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
+        case 126: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 126, 1, false, false, true, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
+        case 256: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 256, 1, false, false, true, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
+        default: return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, false, false, true, 0, PAIR>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
     }
-    return cudaGetLastError();
 }
 
 // RungeKutta4 stages of Model C (deterministic: no noise), axis-aligned or
@@ -824,13 +881,11 @@ cudaError_t launch_strip_oriented(const T* in, T* out, TileArgs g, const typenam
 template <class T, class Ops, int MODE, bool ORIENT>
 cudaError_t launch_strip_rk(const T* in, T* out, TileArgs g, const typename Ops::Params& m, T dt, OrientArgs oa,
                             RkArgs<T> rk, cudaStream_t s) {
-    const bool tail = strip_plan(g, 1 + 3);
-    const dim3 grid = strip_ctas(g), block(256);
+    const bool tail = strip_plan<T>(g, strip_group<T, ORIENT, false>(), 2);
+    const dim3 grid = strip_ctas(g, 2);
     if (tail)
-        modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, true, ORIENT, MODE><<<grid, block, 0, s>>>(in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
-    else
-        modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, false, ORIENT, MODE><<<grid, block, 0, s>>>(in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
-    return cudaGetLastError();
+        return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, true, ORIENT, MODE>, grid, s, in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
+    return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, false, ORIENT, MODE>, grid, s, in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
 }
 
 // kind 2/3/4: single rows, CTAs of 256 threads per SM the register
