@@ -174,10 +174,11 @@ int lg_modelc_initialize_orientations(lg_state* st, int theta_field, const doubl
  * the heat model on `field` (any dimension, FP64) and of Model C (2-D,
  * axis-aligned or multi-grain, FP64 or FP32), deterministic models only (the
  * reference pairs RK4 with NoNoise): a non-zero noise amplitude is refused.
- * Each step is four stage launches, k_i of the stage input written beside
- * y + c_i k_i, the last one applying y += dt/6 k1, dt/3 k2, dt/3 k3, dt/6 k4
- * in the reference's order; FP64 is bit-identical to the reference.  The
- * first run allocates five more arenas of the state's size. */
+ * The axpys y += dt/6 k1, dt/3 k2, dt/3 k3, dt/6 k4 are carried from stage to
+ * stage as a running sum in the reference's order (two launches a step for
+ * heat, four for Model C); FP64 is bit-identical to the reference.  The
+ * first run allocates two (heat; five in 1-D) or three (Model C) more arenas
+ * of the state's size. */
 int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t nsteps, uint32_t flags);
 int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_t nsteps, uint32_t flags);
 /* Heat initial condition of the 96^3 benchmark: sin(2 pi x) sin(2 pi y)

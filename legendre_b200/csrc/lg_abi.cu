@@ -64,8 +64,9 @@ struct lg_state {
     // interior cell on the device (cos block-major, then sin), state dtype
     int theta_field = -1;
     void* orient = nullptr;
-    // RungeKutta4 workspace (allocated at the first RK4 run): k1, k2, k3 and
-    // two stage states, each an arena of the state's layout
+    // RungeKutta4 workspace (allocated at the first RK4 run), each an arena of
+    // the state's layout: the running sum and two stage states (Model C), y + c
+    // k2 and the running sum (heat), or k1, k2, k3 and two stage states (1-D heat)
     void* rk[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
 };
 
@@ -597,7 +598,8 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
              st->orient);
     const int64_t ncells = st->grid->nblocks * st->grid->block[0] * st->grid->block[1];
     // variant = kind + 1000 * rows: kind 0 library default (paired rows on the
-    // work list, 2 CTAs per SM), 1 one thread per cell in reference order, 2/3/4 warp strips with 2/3/4 CTAs per SM, 5/6/7
+    // work list, 2 CTAs per SM), 1 one thread per cell in reference order,
+    // 2/3/4 warp strips with 2/3/4 CTAs per SM, 5/6/7
     // the same with two rows per pass of the row loop, 12..17 those forms as
     // a persistent work list; rows fixes the strip height
     const int kind = variant % 1000 % 10, rows = variant / 1000;
@@ -605,9 +607,6 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
     const bool tile = kind != 1 && lg::modelc_tile_supported(topo);
     const int minb = kind >= 2 ? kind : 5;
     unsigned* work = listed ? reinterpret_cast<unsigned*>(st->d_t + 2) : nullptr;
-    // the run's first step takes its units from a cleared list (each step
-    // clears the other slot's list for the step after it)
-    if (work) LG_CUDA(ctx, cudaMemsetAsync(work + st->tslot, 0, sizeof(unsigned), ctx->stream));
     if (kind == 2 && !tile) return fail(ctx, LG_ERR_INVALID, "the strip kernel needs a 2-D grid");
     auto step = [&]() -> int {
         cudaError_t e;
@@ -902,7 +901,7 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
         return fail(ctx, LG_ERR_INVALID, "RungeKutta4 steps deterministic models only (rk4.rs:15-19): noise must be 0");
     if (nsteps < 0) return fail(ctx, LG_ERR_INVALID, "negative step count");
     cudaSetDevice(ctx->device);
-    int rc = rk_workspace(st, 5);
+    int rc = rk_workspace(st, 3);
     if (rc != LG_OK) return rc;
     if (!st->ghosts_valid) {
         rc = fill_all_ghosts(st);
@@ -925,6 +924,7 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
     const lg::CartTopo topo = topo_of(st->grid);
     const lg::SlabLayout L = layout_of(st, 0);
     const int64_t ncells = st->grid->nblocks * st->grid->block[0] * st->grid->block[1];
+    unsigned* work = reinterpret_cast<unsigned*>(st->d_t + 2);
     const double half_dt = 0.5 * dt, sixth = dt / 6.0, third = dt / 3.0;  // rk4.rs:57, 74-75
     char key[512];
     snprintf(key, sizeof key, "modelc-rk4|%a|%a|%a|%a|%a|dt=%a|orient=%p", p->eps4, p->lambda, p->d_thermal,
@@ -932,28 +932,23 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
     auto step = [&]() -> int {
         const void* y = st->arena[st->cur];
         void* out = st->arena[st->cur ^ 1];
-        void *k1 = st->rk[0], *k2 = st->rk[1], *k3 = st->rk[2], *t0 = st->rk[3], *t1 = st->rk[4];
+        void *acc = st->rk[0], *t0 = st->rk[1], *t1 = st->rk[2];
         const void* stage_in[4] = {y, t0, t1, t0};
         void* stage_out[4] = {t0, t1, t0, out};
-        void* stage_k[3] = {k1, k2, k3};
-        const double stage_c[3] = {half_dt, half_dt, dt};
+        const double stage_c[4] = {half_dt, half_dt, dt, 0.0};
+        const double stage_s[4] = {sixth, third, third, sixth};
         cudaError_t e = cudaSuccess;
         for (int i = 0; i < 4 && e == cudaSuccess; ++i) {
-            const int mode = i < 3 ? 1 : 2;
             if (st->dtype == LG_F64)
                 e = lg::launch_modelc_rk_stage_f64(
-                    mode, static_cast<const double*>(stage_in[i]), static_cast<double*>(stage_out[i]), topo, L, m,
-                    static_cast<const double*>(y), i < 3 ? static_cast<double*>(stage_k[i]) : nullptr,
-                    static_cast<const double*>(k1), static_cast<const double*>(k2), static_cast<const double*>(k3),
-                    i < 3 ? stage_c[i] : 0.0, sixth, third, static_cast<const double*>(st->orient), ncells, st->d_t,
-                    st->tslot, dt, ctx->stream);
+                    i + 1, static_cast<const double*>(stage_in[i]), static_cast<double*>(stage_out[i]), topo, L, m,
+                    static_cast<const double*>(y), static_cast<double*>(acc), stage_c[i], stage_s[i],
+                    static_cast<const double*>(st->orient), ncells, st->d_t, st->tslot, dt, work, ctx->stream);
             else
                 e = lg::launch_modelc_rk_stage_f32(
-                    mode, static_cast<const float*>(stage_in[i]), static_cast<float*>(stage_out[i]), topo, L, m,
-                    static_cast<const float*>(y), i < 3 ? static_cast<float*>(stage_k[i]) : nullptr,
-                    static_cast<const float*>(k1), static_cast<const float*>(k2), static_cast<const float*>(k3),
-                    i < 3 ? stage_c[i] : 0.0, sixth, third, static_cast<const float*>(st->orient), ncells, st->d_t,
-                    st->tslot, dt, ctx->stream);
+                    i + 1, static_cast<const float*>(stage_in[i]), static_cast<float*>(stage_out[i]), topo, L, m,
+                    static_cast<const float*>(y), static_cast<float*>(acc), stage_c[i], stage_s[i],
+                    static_cast<const float*>(st->orient), ncells, st->d_t, st->tslot, dt, work, ctx->stream);
         }
         ctx->launches += 4;
         if (e != cudaSuccess) return cuda_fail(ctx, e, "Model C RK4 stage launch");

@@ -154,13 +154,14 @@ int fill_ghosts(lg_ensemble* e, void* buf) {
 int step_once(lg_ensemble* e, const void* in, void* out, double dt, int slot) {
     const lg::CartTopo topo = topo_of(e);
     const lg::SlabLayout L = layout_of(e);
+    unsigned* work = reinterpret_cast<unsigned*>(e->d_t + 2);
     cudaError_t err;
     if (e->dtype == LG_F64)
         err = lg::launch_modelc_batch_f64((const double*)in, (double*)out, topo, L, e->d_fwd_params, e->d_seeds,
-                                          e->bpi, dt, e->p.noise_amplitude, e->d_t, slot, 0, lg::abi_stream(e->ctx));
+                                          e->bpi, dt, e->p.noise_amplitude, e->d_t, slot, 0, work, lg::abi_stream(e->ctx));
     else
         err = lg::launch_modelc_batch_f32((const float*)in, (float*)out, topo, L, e->d_fwd_params, e->d_seeds, e->bpi,
-                                          dt, e->p.noise_amplitude, e->d_t, slot, 0, lg::abi_stream(e->ctx));
+                                          dt, e->p.noise_amplitude, e->d_t, slot, 0, work, lg::abi_stream(e->ctx));
     lg::abi_count_launch(e->ctx, 1);
     if (err != cudaSuccess) return efail(e, LG_ERR_CUDA, std::string("ensemble step: ") + cudaGetErrorString(err));
     return LG_OK;
@@ -330,8 +331,9 @@ int lg_ensemble_create(lg_ctx* ctx, const int64_t* cells, const int64_t* block, 
         err = cudaMalloc(&e->state[k], state_bytes(e));
         if (err == cudaSuccess) err = cudaMemset(e->state[k], 0, state_bytes(e));
     }
-    if (err == cudaSuccess) err = cudaMalloc(&e->d_t, 2 * sizeof(double));
-    if (err == cudaSuccess) err = cudaMemset(e->d_t, 0, 2 * sizeof(double));
+    // two time slots, then the two work-list counters of the strip kernel
+    if (err == cudaSuccess) err = cudaMalloc(&e->d_t, 3 * sizeof(double));
+    if (err == cudaSuccess) err = cudaMemset(e->d_t, 0, 3 * sizeof(double));
     if (err == cudaSuccess) err = cudaMalloc(&e->d_fwd_params, fwd.size());
     if (err == cudaSuccess) err = cudaMemcpy(e->d_fwd_params, fwd.data(), fwd.size(), cudaMemcpyHostToDevice);
     if (err == cudaSuccess) err = cudaMalloc(&e->d_adj_params, adjp.size());

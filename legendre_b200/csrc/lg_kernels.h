@@ -78,10 +78,11 @@ cudaError_t launch_heat_rk_stage(int mode, const double* in, double* out, const 
 // each face flux is evaluated once and shared by its two cells; `rows` rows
 // of one block per warp (0 = chosen from the grid); `minb` = the form: 2, 3
 // or 4 CTAs per SM the register allocation must allow, 5, 6, 7 the same
-// with two rows per pass of the row loop.  With `work` (two counters, the
-// step's at `slot`) the launch is one wave of CTAs whose warps take further
-// units from the counter; null gives the static grid-stride schedule.  The
-// FP64 results are bit-identical to the reference-order kernel above.
+// with two rows per pass of the row loop.  With `work` (two counters, zero
+// before the launch and after it) a launch of more units than one wave holds
+// is one wave of CTAs whose warps take further units from the counter; null
+// gives the static grid-stride schedule.  The FP64 results are bit-identical
+// to the reference-order kernel above.
 bool modelc_tile_supported(const CartTopo& topo);
 cudaError_t launch_modelc_tile_f64(const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                    const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
@@ -101,21 +102,19 @@ cudaError_t launch_modelc_oriented_f32(const float* in, float* out, const CartTo
                                        const ModelCDev& m, double dt, const NoiseDev& nz, double* tdev, int slot,
                                        const float* trig, int64_t ncells, int rows, unsigned* work, cudaStream_t s);
 
-// One RungeKutta4 stage of Model C without noise (rk4.rs:40-79) on the
-// strip schedule: mode 1 writes the drift of `in` to k and y + c k to out;
-// mode 2 writes (((y + s6 k1) + s3 k2) + s3 k3) + s6 k4 to out.  trig
-// (cos then sin theta0, or null) selects the multi-grain form.  FP64 is
-// bit-identical to the reference's stages.
-cudaError_t launch_modelc_rk_stage_f64(int mode, const double* in, double* out, const CartTopo& topo,
-                                       const SlabLayout& L, const ModelCDev& m, const double* y, double* k,
-                                       const double* k1, const double* k2, const double* k3, double c, double s6,
-                                       double s3, const double* trig, int64_t ncells, double* tdev, int slot,
-                                       double dt, cudaStream_t s);
-cudaError_t launch_modelc_rk_stage_f32(int mode, const float* in, float* out, const CartTopo& topo,
-                                       const SlabLayout& L, const ModelCDev& m, const float* y, float* k,
-                                       const float* k1, const float* k2, const float* k3, double c, double s6,
-                                       double s3, const float* trig, int64_t ncells, double* tdev, int slot,
-                                       double dt, cudaStream_t s);
+// One RungeKutta4 stage (1 to 4) of Model C without noise (rk4.rs:40-79) on
+// the strip schedule: stages 1 to 3 write y + c k to out and carry the step's
+// chain of axpys in acc (stage 1 starts it from y, which is its input); stage
+// 4 writes acc + sum k.  trig (cos then sin theta0, or null) selects the
+// multi-grain form.  FP64 is bit-identical to the reference's stages.
+cudaError_t launch_modelc_rk_stage_f64(int stage, const double* in, double* out, const CartTopo& topo,
+                                       const SlabLayout& L, const ModelCDev& m, const double* y, double* acc, double c,
+                                       double sum, const double* trig, int64_t ncells, double* tdev, int slot,
+                                       double dt, unsigned* work, cudaStream_t s);
+cudaError_t launch_modelc_rk_stage_f32(int stage, const float* in, float* out, const CartTopo& topo,
+                                       const SlabLayout& L, const ModelCDev& m, const float* y, float* acc, double c,
+                                       double sum, const float* trig, int64_t ncells, double* tdev, int slot,
+                                       double dt, unsigned* work, cudaStream_t s);
 
 // Batched instances (an ensemble of independent grids of one geometry):
 // block b of the topology belongs to instance b / bpi, with the parameter
@@ -127,10 +126,10 @@ size_t modelc_record_size_f32();
 void modelc_record_f32(const ModelCDev& m, void* out);
 cudaError_t launch_modelc_batch_f64(const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                     const void* params, const uint64_t* seeds, int bpi, double dt, double amp,
-                                    double* tdev, int slot, int rows, cudaStream_t s);
+                                    double* tdev, int slot, int rows, unsigned* work, cudaStream_t s);
 cudaError_t launch_modelc_batch_f32(const float* in, float* out, const CartTopo& topo, const SlabLayout& L,
                                     const void* params, const uint64_t* seeds, int bpi, double dt, double amp,
-                                    double* tdev, int slot, int rows, cudaStream_t s);
+                                    double* tdev, int slot, int rows, unsigned* work, cudaStream_t s);
 
 // Standard normals of a key array (tests of the generator).
 cudaError_t launch_standard_normal(const uint64_t* keys, double* out, int64_t n, cudaStream_t s);

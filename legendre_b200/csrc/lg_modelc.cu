@@ -33,20 +33,19 @@ cudaError_t launch_modelc_oriented_f64(const double* in, double* out, const Cart
     return launch_strip_oriented<double, OpsExact<double>, false, 2, true>(in, out, g, mc, dt, scale_amp, oa, s);
 }
 
-cudaError_t launch_modelc_rk_stage_f64(int mode, const double* in, double* out, const CartTopo& topo,
-                                       const SlabLayout& L, const ModelCDev& m, const double* y, double* k,
-                                       const double* k1, const double* k2, const double* k3, double c, double s6,
-                                       double s3, const double* trig, int64_t ncells, double* tdev, int slot,
-                                       double dt, cudaStream_t s) {
-    TileArgs g{topo, L, dt, 0, tdev, slot, 0, 0, 0, 0};
+cudaError_t launch_modelc_rk_stage_f64(int stage, const double* in, double* out, const CartTopo& topo,
+                                       const SlabLayout& L, const ModelCDev& m, const double* y, double* acc, double c,
+                                       double sum, const double* trig, int64_t ncells, double* tdev, int slot,
+                                       double dt, unsigned* work, cudaStream_t s) {
+    TileArgs g{topo, L, dt, 0, tdev, slot, 0, 0, 0, 0, work};
     const MC<double> mc = to_mc<double>(m);
     const OrientArgs oa{trig, ncells};
-    const RkArgs<double> rk{y, k, k1, k2, k3, c, s6, s3};
-    if (mode == 1)
-        return trig ? launch_strip_rk<double, OpsExact<double>, 1, true>(in, out, g, mc, dt, oa, rk, s)
-                    : launch_strip_rk<double, OpsExact<double>, 1, false>(in, out, g, mc, dt, oa, rk, s);
-    return trig ? launch_strip_rk<double, OpsExact<double>, 2, true>(in, out, g, mc, dt, oa, rk, s)
-                : launch_strip_rk<double, OpsExact<double>, 2, false>(in, out, g, mc, dt, oa, rk, s);
+    const RkArgs<double> rk{y, acc, (double)c, (double)sum};
+#define LG_RK(MODE)                                                                                \
+    (trig ? launch_strip_rk<double, OpsExact<double>, MODE, true>(in, out, g, mc, (double)dt, oa, rk, s) \
+          : launch_strip_rk<double, OpsExact<double>, MODE, false>(in, out, g, mc, (double)dt, oa, rk, s))
+    return stage == 1 ? LG_RK(1) : stage == 4 ? LG_RK(3) : LG_RK(2);
+#undef LG_RK
 }
 
 size_t modelc_record_size_f64() { return sizeof(MC<double>); }
@@ -54,8 +53,8 @@ void modelc_record_f64(const ModelCDev& m, void* out) { *static_cast<MC<double>*
 
 cudaError_t launch_modelc_batch_f64(const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                     const void* params, const uint64_t* seeds, int bpi, double dt, double amp,
-                                    double* tdev, int slot, int rows, cudaStream_t s) {
-    TileArgs g{topo, L, dt, 0, tdev, slot, rows, 0, 0, 0};
+                                    double* tdev, int slot, int rows, unsigned* work, cudaStream_t s) {
+    TileArgs g{topo, L, dt, 0, tdev, slot, rows, 0, 0, 0, work};
     const BatchArgs bt{params, seeds, bpi};
     const double scale_amp = std::sqrt(dt) * amp;
     if (amp != 0.0) return launch_strip_batch<double, OpsExact<double>, true, 2, true>(in, out, g, bt, dt, scale_amp, s);

@@ -37,7 +37,7 @@
 //
 // Template flags beside the arithmetic: ORIENT steps the multi-grain form
 // (every face's anisotropy in its cell's crystal frame, cos/sin theta0 from a
-// per-state table); MODE 0 is the Euler-Maruyama step, MODE 1 and 2 the
+// per-state table); MODE 0 is the Euler-Maruyama step, MODE 1 to 3 the
 // RungeKutta4 stages (see RkArgs); BATCH serves ensembles; TAIL blocks lower
 // than the row group.
 #pragma once
@@ -61,9 +61,10 @@ struct TileArgs {
     int strips;   // 32-column strips per block
     int chunks;   // row chunks per block
     int64_t units;
-    // persistent work list (null: a static grid-stride schedule): one wave
-    // of CTAs, each warp taking its first unit by position and every further
-    // one from work[slot]; the step clears work[slot ^ 1] for the next step
+    // persistent work list (null: a static grid-stride schedule): one wave of
+    // CTAs, each warp taking its first unit by position and every further one
+    // from work[0].  work[1] counts the warps that are done; the last one sets
+    // both back to zero for the next launch
     unsigned* work;
 };
 
@@ -77,18 +78,17 @@ struct BatchArgs {
     int bpi;
 };
 
-// RungeKutta4 stages (MODE 1, 2; rk4.rs:40-79).  All arenas share the
-// state's slab layout.  MODE 1: k receives the drift of the input, the output
-// is y + c k (y_tmp = y; y_tmp += c k_i).  MODE 2: the output is
-// (((y + s6 k1) + s3 k2) + s3 k3) + s6 k4, k4 the drift of the input.
+// RungeKutta4 stages (MODE 1, 2, 3; rk4.rs:40-79).  All arenas share the
+// state's slab layout.  The step's result is the chain of axpys ((((y + dt/6
+// k1) + dt/3 k2) + dt/3 k3) + dt/6 k4); `acc` carries it from stage to stage in
+// that order, so no k is stored.  MODE 1 (stage 1, the input is y): the output
+// is y + c k, acc = y + s k.  MODE 2 (stages 2 and 3): the output is y + c k,
+// acc += s k.  MODE 3 (stage 4): the output is acc + s k.
 template <class T>
 struct RkArgs {
     const T* y;
-    T* k;
-    const T* k1;
-    const T* k2;
-    const T* k3;
-    T c, s6, s3;
+    T* acc;
+    T c, s;
 };
 
 // Ghost images of a strip's x-edge cells (the block's columns 0 and n0 - 1)
@@ -151,7 +151,7 @@ __device__ __forceinline__ void flush_edges(T* __restrict__ out, const SlabLayou
 }
 
 // The new phi and u of a cell from its drift (kphi, ku): the Euler-Maruyama
-// update (MODE 0) or a RungeKutta4 stage (MODE 1, 2); e0/e1 index the cell's
+// update (MODE 0) or a RungeKutta4 stage (MODE 1 to 3); e0/e1 index the cell's
 // phi/u entries in any arena of the state's layout.
 template <class T, class Ops, bool NOISE, int MODE>
 __device__ __forceinline__ void cell_update(const RkArgs<T>& rk, T dt, T scale_amp, T nval, T kphi, T ku, T p, T uc,
@@ -161,26 +161,25 @@ __device__ __forceinline__ void cell_update(const RkArgs<T>& rk, T dt, T scale_a
         if (NOISE) phin = Ops::add_noise(phin, scale_amp, nval);
         un = Ops::axpy(dt, ku, uc);
     } else if constexpr (MODE == 1) {
-        phin = un = T(0);  // cells that store nothing read nothing either
+        phin = p + rk.c * kphi;
+        un = uc + rk.c * ku;
         if (ok) {
-            rk.k[e0] = kphi;
-            rk.k[e1] = ku;
-            phin = rk.y[e0] + rk.c * kphi;
-            un = rk.y[e1] + rk.c * ku;
+            rk.acc[e0] = p + rk.s * kphi;
+            rk.acc[e1] = uc + rk.s * ku;
         }
     } else {
-        phin = un = T(0);
+        phin = un = T(0);  // cells that store nothing read nothing either
         if (!ok) return;
-        phin = rk.y[e0];
-        phin = phin + rk.s6 * rk.k1[e0];
-        phin = phin + rk.s3 * rk.k2[e0];
-        phin = phin + rk.s3 * rk.k3[e0];
-        phin = phin + rk.s6 * kphi;
-        un = rk.y[e1];
-        un = un + rk.s6 * rk.k1[e1];
-        un = un + rk.s3 * rk.k2[e1];
-        un = un + rk.s3 * rk.k3[e1];
-        un = un + rk.s6 * ku;
+        const T a0 = rk.acc[e0] + rk.s * kphi, a1 = rk.acc[e1] + rk.s * ku;
+        if constexpr (MODE == 2) {
+            phin = rk.y[e0] + rk.c * kphi;
+            un = rk.y[e1] + rk.c * ku;
+            rk.acc[e0] = a0;
+            rk.acc[e1] = a1;
+        } else {
+            phin = a0;
+            un = a1;
+        }
     }
 }
 
@@ -420,13 +419,13 @@ __device__ __forceinline__ void strip_unit(const typename Ops::Params& m, uint64
 // each face in the frame of the cell being updated, shared with the
 // neighbour only where the neighbour's cos/sin theta0 are the same bits,
 // else evaluated again in this cell's frame.
-template <class T, class Ops, bool NOISE, int NX, bool FULL, bool ORIENT = false>
+template <class T, class Ops, bool NOISE, int NX, bool FULL, bool ORIENT = false, int MODE = 0>
 __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, uint64_t seed, int key_block,
                                                 const TileArgs& g, const T* __restrict__ ph,
                                                 const T* __restrict__ uu, T* __restrict__ out, T* __restrict__ po,
                                                 T* __restrict__ uo, const Nbr2& nb, int r0, int r1, int lane,
                                                 int col, bool valid, int last_lane, int cr, bool edge_x, int n0,
-                                                int n1, int sy, double tnow, T dt, T scale_amp, int rs,
+                                                int n1, int sy, double tnow, T dt, T scale_amp, int rs, const RkArgs<T>& rk,
                                                 const T* __restrict__ trig_b = nullptr, int64_t ncells = 0) {
     uint64_t block_key = 0;
     if (NOISE)
@@ -524,6 +523,30 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
         draw();
         const T fb0 = __shfl_sync(kFull, bnd, (j - r0) & 31), fb1 = __shfl_sync(kFull, bnd, (j + 1 - r0) & 31);
         T phin0, phin1, un0, un1, jt1;
+        // rows below rs belong to the unit below (a block's last unit
+        // overlaps it): computed for their faces, stored only once
+        const bool own0 = j >= rs, own1 = j + 1 >= rs;
+        auto update = [&](T kphi0, T ku0, T kphi1, T ku1) {
+            const int64_t e0 = (po - out) + off, e1 = (uo - out) + off;
+            cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nv0, kphi0, ku0, B.b, UB, e0, e1, ok && own0, phin0,
+                                             un0);
+            cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nv1, kphi1, ku1, C.b, UC, e0 + sy, e1 + sy,
+                                             ok && own1, phin1, un1);
+        };
+        if constexpr (MODE >= 2) {  // the stage's other operands of the next pass
+            const int64_t next = j + 3 < n1 ? 2 * (int64_t)sy : 0;
+            const int64_t e0 = (po - out) + off + next, e1 = (uo - out) + off + next;
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.acc + e0));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.acc + e1));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.acc + e0 + sy));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.acc + e1 + sy));
+            if constexpr (MODE == 2) {
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.y + e0));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.y + e1));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.y + e0 + sy));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(rk.y + e1 + sy));
+            }
+        }
         if constexpr (ORIENT) {
             const T q = T(0.25);
             const T jl0 = Ops::oxface(m, c0, s0, B.b - B.a, q * (C.b - A.b + C.a - A.a));
@@ -550,14 +573,7 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             T kphi0, ku0, kphi1, ku1;
             Ops::ocell(m, jr0, jl0, jt0, jbot0, B.b, B.c - B.a, C.b - A.b, c0, s0, UB, ul0, ur0, UC, UA, kphi0, ku0);
             Ops::ocell(m, jr1, jl1, jt1, jbot1, C.b, C.c - C.a, D.b - B.b, c1, s1, UC, ul1, ur1, UD, UB, kphi1, ku1);
-            phin0 = Ops::axpy(dt, kphi0, B.b);
-            phin1 = Ops::axpy(dt, kphi1, C.b);
-            if (NOISE) {
-                phin0 = Ops::add_noise(phin0, scale_amp, nv0);
-                phin1 = Ops::add_noise(phin1, scale_amp, nv1);
-            }
-            un0 = Ops::axpy(dt, ku0, UB);
-            un1 = Ops::axpy(dt, ku1, UC);
+            update(kphi0, ku0, kphi1, ku1);
             cprev = c1;
             sprev = s1;
         } else {
@@ -603,18 +619,8 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
                 Ops::cell(m, fr0, fl0, jt0, jb, B.b, B.c - B.a, C.b - A.b, UB, ul0, ur0, UC, UA, kphi0, ku0);
                 Ops::cell(m, fr1, fl1, jt1, jt0, C.b, C.c - C.a, D.b - B.b, UC, ul1, ur1, UD, UB, kphi1, ku1);
             }
-            phin0 = Ops::axpy(dt, kphi0, B.b);
-            phin1 = Ops::axpy(dt, kphi1, C.b);
-            if (NOISE) {
-                phin0 = Ops::add_noise(phin0, scale_amp, nv0);
-                phin1 = Ops::add_noise(phin1, scale_amp, nv1);
-            }
-            un0 = Ops::axpy(dt, ku0, UB);
-            un1 = Ops::axpy(dt, ku1, UC);
+            update(kphi0, ku0, kphi1, ku1);
         }
-        // rows below rs belong to the unit below (a block's last unit
-        // overlaps it): computed for their faces, stored only once
-        const bool own0 = j >= rs, own1 = j + 1 >= rs;
         store_cell(out, po, uo, off, phin0, un0, ok && own0, own0, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L,
                    nb, eh);
         store_cell(out, po, uo, off + sy, phin1, un1, ok && own1, own1, edge_x, j + 1, r0, n0, n1, col, lane,
@@ -672,9 +678,8 @@ __global__ void __launch_bounds__(256, MINB)
     // writes t + dt to the other slot (simulation.rs:285), so a captured
     // sequence of steps needs no host-side time.
     const double tnow = g.tdev[g.slot];
-    if (MODE != 1 && blockIdx.x == 0 && threadIdx.x == 0) {
+    if ((MODE == 0 || MODE == 3) && blockIdx.x == 0 && threadIdx.x == 0) {
         g.tdev[g.slot ^ 1] = tnow + g.dt64;
-        if (g.work) g.work[g.slot ^ 1] = 0u;
     }
 
     while (unit < g.units) {
@@ -701,18 +706,18 @@ __global__ void __launch_bounds__(256, MINB)
         T* po = out + slab_base(g.L, b, 0);
         T* uo = out + slab_base(g.L, b, 1);
         if constexpr (PAIR) {
-            static_assert(MODE == 0 && !TAIL && !(ORIENT && BATCH), "the paired rows serve the Euler-Maruyama step");
+            static_assert(!TAIL && !(ORIENT && BATCH), "the paired rows need whole groups");
             if constexpr (BATCH) {
                 const int inst = b / bt.bpi;
                 const typename Ops::Params mi = static_cast<const typename Ops::Params*>(bt.params)[inst];
-                strip_unit_pair<T, Ops, NOISE, NX, FULL>(mi, bt.seeds[inst], b - inst * bt.bpi, g, ph, uu, out, po, uo,
+                strip_unit_pair<T, Ops, NOISE, NX, FULL, false, MODE>(mi, bt.seeds[inst], b - inst * bt.bpi, g, ph, uu, out, po, uo,
                                                          nb, r0, r1, lane, col, valid, last_lane, cr, edge_x, n0, n1,
-                                                         sy, tnow, dt, scale_amp, rs);
+                                                         sy, tnow, dt, scale_amp, rs, rk);
             } else {
                 const T* trig_b = ORIENT ? static_cast<const T*>(oa.trig) + (int64_t)b * n0 * n1 : nullptr;
-                strip_unit_pair<T, Ops, NOISE, NX, FULL, ORIENT>(m0, g.seed, b, g, ph, uu, out, po, uo, nb, r0, r1,
+                strip_unit_pair<T, Ops, NOISE, NX, FULL, ORIENT, MODE>(m0, g.seed, b, g, ph, uu, out, po, uo, nb, r0, r1,
                                                                  lane, col, valid, last_lane, cr, edge_x, n0, n1, sy,
-                                                                 tnow, dt, scale_amp, rs, trig_b, oa.ncells);
+                                                                 tnow, dt, scale_amp, rs, rk, trig_b, oa.ncells);
             }
         } else if constexpr (BATCH) {
             const int inst = b / bt.bpi;
@@ -730,7 +735,7 @@ __global__ void __launch_bounds__(256, MINB)
         }
         if (g.work) {  // the next unit of the list
             unsigned n = 0;
-            if (lane == 0) n = atomicAdd(g.work + g.slot, 1u);
+            if (lane == 0) n = atomicAdd(g.work, 1u);
             unit = first_listed + (int64_t)__shfl_sync(kFull, n, 0);
         } else {
             unit += first_listed;
@@ -739,6 +744,10 @@ __global__ void __launch_bounds__(256, MINB)
             su.decode(g, unit);
             nb.load(topo, su.b);
         }
+    }
+    if (g.work && lane == 0 && atomicAdd(g.work + 1, 1u) == gridDim.x * wpc - 1) {
+        g.work[0] = 0u;
+        g.work[1] = 0u;
     }
 }
 
@@ -877,15 +886,21 @@ cudaError_t launch_strip_oriented(const T* in, T* out, TileArgs g, const typenam
 }
 
 // RungeKutta4 stages of Model C (deterministic: no noise), axis-aligned or
-// multi-grain, any block width
+// multi-grain, on the paired rows; common block widths get a compile-time row
+// stride
 template <class T, class Ops, int MODE, bool ORIENT>
 cudaError_t launch_strip_rk(const T* in, T* out, TileArgs g, const typename Ops::Params& m, T dt, OrientArgs oa,
                             RkArgs<T> rk, cudaStream_t s) {
-    const bool tail = strip_plan<T>(g, strip_group<T, ORIENT, false>(), 2);
+    const bool tail = strip_plan<T>(g, strip_group<T, ORIENT, true>(), 2);
     const dim3 grid = strip_ctas(g, 2);
-    if (tail)
-        return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, true, ORIENT, MODE>, grid, s, in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
-    return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, false, ORIENT, MODE>, grid, s, in, out, g, m, dt, T(0), BatchArgs{}, oa, rk);
+    const BatchArgs nob{};
+    if (tail)  // blocks of one row
+        return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, true, ORIENT, MODE>, grid, s, in, out, g, m, dt, T(0), nob, oa, rk);
+    switch (g.topo.n[0]) {
+        case 126: return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 126, 1, false, false, ORIENT, MODE, true>, grid, s, in, out, g, m, dt, T(0), nob, oa, rk);
+        case 128: return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 128, 1, false, false, ORIENT, MODE, true>, grid, s, in, out, g, m, dt, T(0), nob, oa, rk);
+        default: return strip_launch(modelc_strip_kernel<T, Ops, false, 2, 0, 1, false, false, ORIENT, MODE, true>, grid, s, in, out, g, m, dt, T(0), nob, oa, rk);
+    }
 }
 
 // kind 2/3/4: single rows, CTAs of 256 threads per SM the register
