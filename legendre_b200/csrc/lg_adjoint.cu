@@ -483,6 +483,8 @@ __global__ void __launch_bounds__(256) adjoint_strip_kernel(const T* __restrict_
                                                             double* __restrict__ acc, int rows, int strips,
                                                             int chunks, unsigned long long* __restrict__ work,
                                                             unsigned long long work_base) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     const int lane = threadIdx.x & 31;
     const int64_t units = g.ninst * strips * chunks;
     const int64_t first_listed = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -790,6 +792,16 @@ cudaError_t launch_adjoint(const T* x, const T* lam_in, T* lam_out, const void* 
     return cudaGetLastError();
 }
 
+// resident CTAs of the strip kernel per SM
+template <class T>
+int adjoint_strip_ctas() {
+    static const int per_sm = [] {
+        int n = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_strip_kernel<T>, 256, 0) != cudaSuccess) n = 1;
+        return std::max(n, 1);
+    }();
+    return per_sm;
+}
 
 // With a work list the grid is one wave of resident CTAs and each warp
 // takes its next unit from the counter when it finishes one, so the strips
@@ -800,22 +812,24 @@ cudaError_t launch_adjoint(const T* x, const T* lam_in, T* lam_out, const void* 
 template <class T>
 cudaError_t launch_adjoint_strip(const T* x, const T* lam_in, T* lam_out, const void* prm, const Geo& g, double dt,
                                  double* acc, unsigned long long* work, unsigned long long base, cudaStream_t s) {
-    const int strips = adjoint_strips(g), rows = adjoint_strip_rows(g);
+    const int strips = adjoint_strips(g), rows = adjoint_strip_rows(sizeof(T) == 8 ? 0 : 1, g);
     const int chunks = (g.N1 + rows - 1) / rows;
     const int64_t units = g.ninst * strips * chunks;
     int64_t grid = std::min<int64_t>((units + 7) / 8, (int64_t)1 << 30);
-    if (work) {
-        static const int per_sm = [] {
-            int n = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, adjoint_strip_kernel<T>, 256, 0) != cudaSuccess)
-                n = 1;
-            return std::max(n, 1);
-        }();
-        grid = std::min<int64_t>(grid, (int64_t)lg::device_sm_count() * per_sm);
-    }
-    adjoint_strip_kernel<T><<<(unsigned)grid, 256, 0, s>>>(x, lam_in, lam_out, static_cast<const AdjParams<T>*>(prm),
-                                                           g, (T)dt, acc, rows, strips, chunks, work, base);
-    return cudaGetLastError();
+    if (work) grid = std::min<int64_t>(grid, (int64_t)lg::device_sm_count() * adjoint_strip_ctas<T>());
+    // programmatic dependent launch: the next step's CTAs start while this
+    // step's last ones finish, and wait before they touch the state
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(256);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, adjoint_strip_kernel<T>, x, lam_in, lam_out,
+                              static_cast<const AdjParams<T>*>(prm), g, (T)dt, acc, rows, strips, chunks, work, base);
 }
 
 }  // namespace
@@ -824,19 +838,37 @@ int adjoint_tile_rows(int dtype) { return dtype == 0 ? 8 : 16; }
 
 int adjoint_strips(const Geo& g) { return (g.N0 + SW - 1) / SW; }
 
-// rows per strip unit: the whole instance height, halved while the launch
-// would hold fewer units than 15 warps per SM, most of one wave of 16 (down
-// to 16 rows).  Each unit completes two rows beyond the ones it gathers, so
-// tall units waste least; the work list evens out the rest (on 256
-// instances of 256^2, 9 x 256 = 2304 units of the whole height, 97 % of a
-// wave, ran the gradient 0.5 % faster than 128-row units, which ran it
-// 1.6 % faster than 64-row ones)
-int adjoint_strip_rows(const Geo& g) {
+// Rows per strip unit.  FP64: the whole instance height or a halving of it
+// (down to 4 rows), whichever makes the launch shortest: a unit completes two
+// rows beyond the ones it gathers and spends about four rows' time on
+// starting, and a row takes the same time until the resident warps are all
+// busy; from there on the units queue.  FP32: halved while the launch would
+// hold fewer units than 15 warps per SM, most of one wave of 16 (down to 16
+// rows).  There the contracted sums of a unit's first rows round as they do
+// nowhere else, so moving the boundaries moves the gradients' last bits (2e-8
+// relative); 8-row units would run 32 instances of 128^2 in 24.5 instead of
+// 28 us a step.  On 256 instances of 256^2 whole instances (2304 units, 97 %
+// of a wave) are best.
+int adjoint_strip_rows(int dtype, const Geo& g) {
     const int strips = adjoint_strips(g);
-    const int64_t wave = (int64_t)lg::device_sm_count() * 15;
-    int rows = std::max(1, g.N1);
-    while (rows > 16 && g.ninst * strips * ((g.N1 + rows - 1) / rows) < wave) rows = (rows + 1) / 2;
-    return rows;
+    if (dtype != 0) {
+        const int64_t wave = (int64_t)lg::device_sm_count() * 15;
+        int rows = std::max(1, g.N1);
+        while (rows > 16 && g.ninst * strips * ((g.N1 + rows - 1) / rows) < wave) rows = (rows + 1) / 2;
+        return rows;
+    }
+    const double slots = (double)lg::device_sm_count() * 8 * adjoint_strip_ctas<double>();
+    int best = std::max(1, g.N1);
+    double best_cost = 0.0;
+    for (int rows = best;; rows = (rows + 1) / 2) {
+        const double units = (double)g.ninst * strips * ((g.N1 + rows - 1) / rows);
+        const double cost = (rows + 6) * std::max(1.0, units / slots);
+        if (best_cost == 0.0 || cost < best_cost) {
+            best_cost = cost;
+            best = rows;
+        }
+        if (rows <= 4) return best;
+    }
 }
 
 cudaError_t launch_adjoint_step(int dtype, int kernel, const void* x, const void* lam_in, void* lam_out,
@@ -872,7 +904,7 @@ int64_t loss_items(const Geo& g) { return (int64_t)g.ninst * ((g.N0 + TW - 1) / 
 
 int64_t adjoint_items(int dtype, int kernel, const Geo& g) {
     if (kernel == kAdjointStrip) {
-        const int rows = adjoint_strip_rows(g);
+        const int rows = adjoint_strip_rows(dtype, g);
         return g.ninst * adjoint_strips(g) * ((g.N1 + rows - 1) / rows);
     }
     const int th = adjoint_tile_rows(dtype);

@@ -36,7 +36,7 @@ constexpr int kAdjointStrip = 0, kAdjointTile = 1;
 
 int adjoint_tile_rows(int dtype);
 int adjoint_strips(const Geo& g);
-int adjoint_strip_rows(const Geo& g);
+int adjoint_strip_rows(int dtype, const Geo& g);
 // work items (tiles or strip units); the accumulator holds 3 doubles per item
 int64_t adjoint_items(int dtype, int kernel, const Geo& g);
 int64_t loss_items(const Geo& g);                // tiles of the loss kernel; one double each
