@@ -366,11 +366,29 @@ __device__ __forceinline__ void restrict_ops(double* C, const double* F, const R
     }
 }
 
-__global__ void amr_restrict_kernel(double* C, const double* F, const RestrictOp* __restrict__ ops, int64_t nops,
-                                    int r, double inv, int f0, int f1) {
+// One covered cell and field a thread (blockIdx.y: the field).  The cell's op
+// is read before the dependency wait; ratio 2 issues its four loads at once.
+__global__ void __launch_bounds__(256) amr_restrict_kernel(double* C, const double* F,
+                                                           const RestrictOp* __restrict__ ops, int64_t nops, int r,
+                                                           double inv, int f0, int f1) {
     pdl_release();
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    RestrictOp op{};
+    if (i < nops) op = ops[i];
     pdl_wait();
-    restrict_ops(C, F, ops, nops, r, inv, f0, f1);
+    if (i >= nops) return;
+    for (int f = f0 + (int)blockIdx.y; f < f1; f += gridDim.y) {
+        const double* src = F + op.f + (int64_t)f * op.fstride;
+        double sum = 0.0;
+        if (r == 2) {
+            const double a = src[0], b = src[1], c = src[op.fsy], d = src[1 + op.fsy];
+            sum = (((sum + a) + b) + c) + d;
+        } else {
+            for (int ky = 0; ky < r; ++ky)
+                for (int kx = 0; kx < r; ++kx) sum += src[kx + ky * op.fsy];
+        }
+        C[op.c + (int64_t)f * op.cstride] = sum * inv;
+    }
 }
 
 // launch with the programmatic-dependent-launch attribute (see pdl_release)
@@ -651,26 +669,31 @@ std::pair<int64_t, int64_t> level_range(const lg_amr_sim* s, int level) {
     return {s->plans.blocks[b0].off, last.off + last.stride * s->nfields};
 }
 
-// Tile shape per level.  A level with enough cells to fill the GPU several
-// times over is throughput-bound: 32-row tiles, four rows per warp, so that
-// each face flux is shared down a warp's rows.  A sparse fine level is
-// latency-bound (its launch is one short wave): tiles of at most 8 rows with
-// one row per warp, the tallest that still gives two tiles per SM.
+// Tile shape per level: the one whose waves of resident CTAs take least time.
+// A CTA spends about three rows' time on staging its window and starting,
+// then a row's time on each of a warp's rows; 64 registers a thread leave 32
+// warps per SM.  (A fine level of 608 tiles of 8 rows, one row a warp, was 16
+// tiles over a wave of 592; 1107 tiles of 4 rows fit one of 1184.  512^2 base
+// and three levels, 106 launches a coarse step: 0.77 -> 0.55 ms.)
 std::vector<TileShape> choose_tile_shapes(const lg::amr::Layout& g) {
-    const int kSMs = lg::device_sm_count();
+    const int64_t kSMs = lg::device_sm_count();
     std::vector<TileShape> shapes(g.max_levels(), TileShape{lg::amr::kTile, 4});
+    const TileShape candidates[] = {{32, 4}, {16, 2}, {8, 1}, {4, 1}, {2, 1}, {1, 1}};
     for (int l = 0; l < g.num_levels(); ++l) {
-        int64_t cells = 0;
-        for (uint32_t b = g.level_start[l]; b < g.level_start[l + 1]; ++b) cells += g.patches[b].bx.cells();
-        if (cells >= (int64_t)kSMs * 2048) continue;
-        for (int r : {8, 4, 2, 1}) {
+        double best = 0.0;
+        for (const TileShape& t : candidates) {
             int64_t tiles = 0;
             for (uint32_t b = g.level_start[l]; b < g.level_start[l + 1]; ++b) {
                 const auto& bx = g.patches[b].bx;
-                tiles += ((bx.extent(0) + lg::amr::kTile - 1) / lg::amr::kTile) * ((bx.extent(1) + r - 1) / r);
+                tiles += ((bx.extent(0) + lg::amr::kTile - 1) / lg::amr::kTile) *
+                         ((bx.extent(1) + t.rows - 1) / t.rows);
             }
-            shapes[l] = TileShape{r, 1};
-            if (tiles >= 2 * kSMs) break;
+            const int64_t slots = kSMs * (32 / (t.rows / t.rows_per_warp));
+            const double cost = (double)std::max<int64_t>(1, (tiles + slots - 1) / slots) * (3 + t.rows_per_warp);
+            if (best == 0.0 || cost < best) {
+                best = cost;
+                shapes[l] = t;
+            }
         }
     }
     return shapes;
@@ -838,7 +861,8 @@ int launch_restrict(lg_amr_sim* s, int fine, int f0, int f1) {
     if (b == a) return LG_OK;
     const int r = (int)s->layout.ratios[fine - 1];
     const double inv = 1.0 / ((double)r * (double)r);
-    AMR_CUDA(s, launch_pdl(amr_restrict_kernel, dim3(grid_for(b - a, 256)), dim3(256), lg::abi_stream(s->ctx),
+    AMR_CUDA(s, launch_pdl(amr_restrict_kernel, dim3((unsigned)((b - a + 255) / 256), (unsigned)(f1 - f0)), dim3(256),
+                           lg::abi_stream(s->ctx),
                            s->arena[s->cur[fine - 1]], (const double*)s->arena[s->cur[fine]],
                            (const RestrictOp*)(s->tab.restrict_ops + a), (int64_t)(b - a), r, inv, f0, f1));
     lg::abi_count_launch(s->ctx, 1);
