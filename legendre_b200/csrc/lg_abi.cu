@@ -57,6 +57,10 @@ struct lg_state {
     double* d_t = nullptr;    // two time slots
     int tslot = 0;
     double t = 0.0;
+    // the device's time slot `tslot` holds exactly dev_t (the kernels advance
+    // it by the host's own additions), so a run that starts there copies nothing
+    double dev_t = 0.0;
+    bool dev_t_known = false;
     int64_t step_index = 0;
     bool ghosts_valid = false;
     std::map<std::string, GraphEntry> graphs;
@@ -202,11 +206,29 @@ std::string tune_key(const lg_state* st, bool noise) {
            std::to_string(g->nblocks) + "|" + std::to_string(st->dtype) + "|" + (noise ? "n" : "q");
 }
 
+// The device time slot of a Model C run starts from the host's time; it is
+// unknown until the run's kernels have all been launched (see advance_model_c)
+int set_device_time(lg_state* st) {
+    const bool there = st->dev_t_known && memcmp(&st->dev_t, &st->t, sizeof(double)) == 0;
+    st->dev_t_known = false;
+    if (!there)
+        LG_CUDA(st->ctx, cudaMemcpyAsync(st->d_t + st->tslot, &st->t, sizeof(double), cudaMemcpyHostToDevice,
+                                         st->ctx->stream));
+    return LG_OK;
+}
+
 // Host-side time bookkeeping of `steps` steps: t += dt each
 // (simulation.rs:285-286), the same IEEE additions the kernels perform.
 void advance_time(lg_state* st, double dt, int64_t steps) {
     for (int64_t s = 0; s < steps; ++s) st->t += dt;
     st->step_index += steps;
+}
+
+// after a Model C run: its kernels left the same time in the device's slot
+void advance_model_c(lg_state* st, double dt, int64_t steps) {
+    advance_time(st, dt, steps);
+    st->dev_t = st->t;
+    st->dev_t_known = true;
 }
 
 }  // namespace
@@ -535,6 +557,7 @@ int lg_heat_fe_run(lg_state* st, int field, double kappa, double dt, int64_t nst
         if (e != cudaSuccess) return cuda_fail(ctx, e, "heat step launch");
         st->cur ^= 1;
         st->tslot ^= 1;
+        st->dev_t_known = false;  // the heat kernels keep no device time
         return LG_OK;
     };
     // double steps, then single ones.  Fields that no launch writes keep to
@@ -584,8 +607,7 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
     nz.on = p->noise_amplitude != 0.0 ? 1 : 0;
     nz.seed = seed;
     nz.amp = p->noise_amplitude;
-    // the device time slot starts from the host's time
-    LG_CUDA(ctx, cudaMemcpyAsync(st->d_t + st->tslot, &st->t, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    if (int rc = set_device_time(st); rc != LG_OK) return rc;
     const lg::CartTopo topo = topo_of(st->grid);
     const lg::SlabLayout L = layout_of(st, 0);
     if (variant == 0) {  // the autotuned choice for this shape, if any
@@ -638,7 +660,7 @@ int lg_modelc_em_run(lg_state* st, const lg_modelc_params* p, double dt, uint64_
     };
     int rc = run_steps(st, key, nsteps, flags, step);
     if (rc != LG_OK) return rc;
-    advance_time(st, dt, nsteps);
+    advance_model_c(st, dt, nsteps);
     return LG_OK;
 }
 
@@ -679,6 +701,7 @@ int lg_modelc_autotune(lg_state* st, const lg_modelc_params* p, double dt, uint6
         st->cur = cur0;
         st->tslot = slot0;
         st->t = t0;
+        st->dev_t_known = false;
         rc = lg_modelc_em_run(st, p, dt, seed, 2, v, 0);  // warm-up
         if (rc != LG_OK) return -1.0f;
         cudaEventRecord(e0, ctx->stream);
@@ -734,6 +757,7 @@ int lg_modelc_autotune(lg_state* st, const lg_modelc_params* p, double dt, uint6
     st->cur = cur0;
     st->tslot = slot0;
     st->t = t0;
+    st->dev_t_known = false;
     st->step_index = k0;
     if (rc != LG_OK) return rc;
     ctx->tuned[key] = best;
@@ -866,6 +890,7 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
             if (e != cudaSuccess) return cuda_fail(ctx, e, "heat RK4 launch");
             st->cur ^= 1;
             st->tslot ^= 1;
+            st->dev_t_known = false;  // the heat kernels keep no device time
             return LG_OK;
         }
         e = lg::launch_heat_rk_stage(1, y, t0, y, k1, nullptr, nullptr, nullptr, topo, L, field, kappa,
@@ -883,6 +908,7 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
         if (e != cudaSuccess) return cuda_fail(ctx, e, "heat RK4 stage launch");
         st->cur ^= 1;
         st->tslot ^= 1;
+        st->dev_t_known = false;
         return LG_OK;
     };
     rc = run_steps(st, key, nsteps, flags, step);
@@ -920,7 +946,8 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
     m.inv_h2_flux = 1.0 / (st->grid->spacing[0] * st->grid->spacing[1]);
     m.inv_h2[0] = 1.0 / (st->grid->spacing[0] * st->grid->spacing[0]);
     m.inv_h2[1] = 1.0 / (st->grid->spacing[1] * st->grid->spacing[1]);
-    LG_CUDA(ctx, cudaMemcpyAsync(st->d_t + st->tslot, &st->t, sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+    rc = set_device_time(st);
+    if (rc != LG_OK) return rc;
     const lg::CartTopo topo = topo_of(st->grid);
     const lg::SlabLayout L = layout_of(st, 0);
     const int64_t ncells = st->grid->nblocks * st->grid->block[0] * st->grid->block[1];
@@ -958,7 +985,7 @@ int lg_modelc_rk4_run(lg_state* st, const lg_modelc_params* p, double dt, int64_
     };
     rc = run_steps(st, key, nsteps, flags, step);
     if (rc != LG_OK) return rc;
-    advance_time(st, dt, nsteps);
+    advance_model_c(st, dt, nsteps);
     return LG_OK;
 }
 

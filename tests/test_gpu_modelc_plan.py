@@ -50,3 +50,34 @@ def test_multi_grain_steps_one_by_one(sched, cells, block, dtype):
     got = _run(sched, cells, block, 0.02, True, [(7, False), (8, True)], 0, dtype)
     ref = _run(sched, cells, block, 0.02, True, [(1, False)] * 15, 0, dtype)
     assert all(np.array_equal(a, b) for a, b in zip(got, ref))
+
+
+def test_noise_follows_the_state_time(sched):
+    # the device keeps the time between runs; a run after set_time, after an
+    # autotune or on a fresh state starts from the state's own time
+    def sim_of():
+        grid = L.CartesianGrid([64, 32], [32, 16], [0.0, 0.0], [H, H])
+        return L.Simulation(grid, L.FiniteVolume(), L.ModelC(0.05, 3.19, 0.02), L.EulerMaruyama(9), sched,
+                            L.CudaAllocator("f64"))
+
+    a = sim_of()
+    rng = np.random.default_rng(2)
+    fields = [with_ghosts(0.1 * rng.standard_normal((4, 16, 32)), 1) for _ in range(2)]
+    for f in (0, 1):
+        a.state.upload(f, fields[f])
+    t = None
+    for leg, (start, steps) in enumerate([(None, 3), (None, 2), (5.25, 1), (0.0, 4), (None, 3)]):
+        if start is not None:
+            a.state.set_time(start, 0)
+        if leg == 4:
+            a.autotune(0.008, trial_steps=1)
+        t, k = a.state.time
+        b = sim_of()
+        for f in (0, 1):
+            b.state.upload(f, fields[f])
+        b.state.set_time(t, k)
+        for s in (a, b):
+            s.run(0.008, steps, variant=5)
+        assert a.state.time == b.state.time
+        fields = [a.state.download(f) for f in (0, 1)]
+        assert all(np.array_equal(x, b.state.download(f)) for f, x in enumerate(fields))
