@@ -614,6 +614,8 @@ struct lg_amr_sim {
     int coop_grid[2] = {0, 0};  // per model kind (noise-free / noisy) once measured
     std::vector<double> host_old, host_new;  // host staging of whole states (get/set)
     std::vector<TileShape> tile_shapes;      // per level
+    char* h_tab = nullptr;  // page-locked staging of upload_tables
+    size_t h_tab_cap = 0;
     // regrid migration on the device: the old state's image and the old
     // hierarchy's patch tables (grow-only)
     double* d_mig_old = nullptr;
@@ -727,9 +729,20 @@ int upload_tables(lg_amr_sim* s, const lg::amr::Plans& P, const lg::amr::Layout&
     const size_t o_units = reserve(P.units.size() * sizeof(Unit));
     const size_t o_tiles = reserve(P.tiles.size() * sizeof(lg::amr::Tile));
     const size_t o_tfill = reserve(P.tile_fill.size() * sizeof(GhostOp));
-    std::vector<char> blob(std::max<size_t>(off, 256), 0);
+    // packed into page-locked memory that the simulation keeps (every copy
+    // from it ends before this function returns)
+    off = std::max<size_t>(off, 256);
+    if (off > s->h_tab_cap) {
+        cudaFreeHost(s->h_tab);
+        s->h_tab = nullptr;
+        s->h_tab_cap = 0;
+        const size_t cap = off + off / 2;
+        AMR_CUDA(s, cudaMallocHost(&s->h_tab, cap));
+        s->h_tab_cap = cap;
+    }
+    char* const blob = s->h_tab;
     auto put = [&](size_t o, const void* src, size_t bytes) {
-        if (bytes) std::memcpy(blob.data() + o, src, bytes);
+        if (bytes) std::memcpy(blob + o, src, bytes);
     };
     put(o_blocks, P.blocks.data(), P.blocks.size() * sizeof(BlockDesc));
     put(o_lo, lo.data(), lo.size() * sizeof(int64_t));
@@ -738,15 +751,15 @@ int upload_tables(lg_amr_sim* s, const lg::amr::Plans& P, const lg::amr::Layout&
     put(o_units, P.units.data(), P.units.size() * sizeof(Unit));
     put(o_tiles, P.tiles.data(), P.tiles.size() * sizeof(lg::amr::Tile));
     put(o_tfill, P.tile_fill.data(), P.tile_fill.size() * sizeof(GhostOp));
-    if (blob.size() > T.cap) {
+    if (off > T.cap) {
         cudaFree(T.d);
         T = Tables{};
-        const size_t cap = blob.size() + blob.size() / 4;
+        const size_t cap = off + off / 4;
         AMR_CUDA(s, cudaMalloc(&T.d, cap));
         T.cap = cap;
     }
     cudaStream_t st = lg::abi_stream(s->ctx);
-    AMR_CUDA(s, cudaMemcpyAsync(T.d, blob.data(), blob.size(), cudaMemcpyHostToDevice, st));
+    AMR_CUDA(s, cudaMemcpyAsync(T.d, blob, off, cudaMemcpyHostToDevice, st));
     AMR_CUDA(s, cudaStreamSynchronize(st));
     T.blocks = (BlockDesc*)(T.d + o_blocks);
     T.lo = (int64_t*)(T.d + o_lo);
@@ -1326,14 +1339,17 @@ __device__ double mig_sample(const MigArgs& a, int level, int64_t x, int64_t y, 
     }
 }
 
+// A sample is a chain of dependent table look-ups, so the cells of a block
+// and its fields are spread over several CTAs (y: runs of cells, z: fields):
+// 317 blocks of three levels 200 to 330 us with one CTA a block.
 __global__ void __launch_bounds__(256) amr_migrate_kernel(MigArgs a) {
+    const int f = blockIdx.z;
     for (int bi = blockIdx.x; bi < a.nblocks; bi += gridDim.x) {
         const MigBlock B = a.blocks[bi];
-        for (int c = threadIdx.x; c < B.nx * B.ny; c += blockDim.x) {
+        for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < B.nx * B.ny; c += gridDim.y * blockDim.x) {
             const int i = c % B.nx, j = c / B.nx;
             const int64_t o = B.off + (i + 1) + (int64_t)(j + 1) * (B.nx + 2);
-            for (int f = 0; f < a.nfields; ++f)
-                a.out[o + (int64_t)f * B.stride] = mig_sample<kMaxDepth - 1>(a, B.level, B.lo[0] + i, B.lo[1] + j, f);
+            a.out[o + (int64_t)f * B.stride] = mig_sample<kMaxDepth - 1>(a, B.level, B.lo[0] + i, B.lo[1] + j, f);
         }
     }
 }
@@ -1478,7 +1494,7 @@ int maybe_regrid(lg_amr_sim* s) {
         AMR_CUDA(s, cudaMemsetAsync(s->arena[keep] + l0, 0, (size_t)(np.arena_elems - l0) * sizeof(double), st));
         ma.out = s->arena[keep];
         if (ma.nblocks > 0) {
-            amr_migrate_kernel<<<(unsigned)std::min(ma.nblocks, 65535), 256, 0, st>>>(ma);
+            amr_migrate_kernel<<<dim3((unsigned)std::min(ma.nblocks, 65535), 4, (unsigned)ma.nfields), 256, 0, st>>>(ma);
             lg::abi_count_launch(s->ctx, 1);
             AMR_CUDA(s, cudaGetLastError());
         }
@@ -1597,6 +1613,7 @@ int lg_amr_sim_destroy(lg_amr_sim* s) {
     cudaFree(s->d_mig_old);
     cudaFree(s->d_mig_tab);
     cudaFree(s->d_mig_err);
+    cudaFreeHost(s->h_tab);
     delete s;
     return LG_OK;
 }

@@ -383,6 +383,13 @@ Plans build_plans(const Layout& g, int nfields, int unit_cells, int first_level,
         P.blocks.push_back(d);
     }
     P.arena_elems = off;
+    // room for every ring entry (a tile's window repeats few of them)
+    size_t ring = 0;
+    for (uint32_t b = first_level < g.num_levels() ? g.level_start[first_level] : (uint32_t)g.num_blocks();
+         b < (uint32_t)g.num_blocks(); ++b)
+        ring += 2 * (size_t)(P.blocks[b].nx + P.blocks[b].ny) + 4;
+    P.fill.reserve(ring);
+    P.tile_fill.reserve(ring + ring / 4);
     auto slab_off = [&](int b, int64_t i, int64_t j) { return (int)((i + 1) + (j + 1) * (P.blocks[b].nx + 2)); };
 
     // ghost fill (intergrid.rs:267-351, ghost width 1), and the tiles of
@@ -395,12 +402,18 @@ Plans build_plans(const Layout& g, int nfields, int unit_cells, int first_level,
         for (uint32_t pb = g.level_start[level]; pb < g.level_start[level + 1]; ++pb) {
             const Box& bx = g.patches[pb].bx;
             const size_t ring0 = P.fill.size();
+            // consecutive ring cells mostly lie in the same source patch
+            auto find = [&](int l, int64_t x, int64_t y, int& last) {
+                if (last < 0 || !g.patches[(size_t)last].bx.contains(x, y)) last = g.find(l, x, y);
+                return last;
+            };
+            int near = -1, below[4] = {-1, -1, -1, -1};
             auto visit = [&](int64_t x, int64_t y) {
                 GhostOp op{};
                 op.dst = P.blocks[pb].off + slab_off((int)pb, x - bx.lo[0], y - bx.lo[1]);
                 op.dst_stride = (int32_t)P.blocks[pb].stride;
                 const int64_t tx = reflect(x, dom.lo[0], dom.hi[0]), ty = reflect(y, dom.lo[1], dom.hi[1]);
-                const int src = g.find(level, tx, ty);
+                const int src = find(level, tx, ty, near);
                 if (src >= 0) {
                     const Box& sb = g.patches[src].bx;
                     op.n = 0;
@@ -432,7 +445,7 @@ Plans build_plans(const Layout& g, int nfields, int unit_cells, int first_level,
                         }
                         if (weight == 0.0) continue;
                         for (int d = 0; d < 2; ++d) cc[d] = reflect(cc[d], cd.lo[d], cd.hi[d]);
-                        const int q = g.find(level - 1, cc[0], cc[1]);
+                        const int q = find(level - 1, cc[0], cc[1], below[corner]);
                         if (q < 0) {  // the reference panics: proper nesting guarantees a donor
                             P.error = "no coarse donor for prolongation at level " + std::to_string(level);
                             continue;
@@ -466,15 +479,23 @@ Plans build_plans(const Layout& g, int nfields, int unit_cells, int first_level,
                     t.w = std::min(kTile, nx - x0);
                     t.h = std::min(th, ny - y0);
                     t.fill0 = (int)P.tile_fill.size();
-                    for (size_t k = ring0; k < P.fill.size(); ++k) {
-                        const int toff = (int)(P.fill[k].dst - P.blocks[pb].off);
-                        const int i = toff % (nx + 2) - 1, j = toff / (nx + 2) - 1;
-                        const int c = i - (x0 - 1), r = j - (y0 - 1);
-                        if (c < 0 || c > t.w + 1 || r < 0 || r > t.h + 1) continue;
-                        GhostOp op = P.fill[k];
-                        op.dst = c + r * (t.w + 2);
+                    // the ring entries inside the window, in ring order (left and
+                    // right columns upwards, bottom and top rows with corners)
+                    const int j0 = std::max(0, y0 - 1), j1 = std::min(ny - 1, y0 + t.h);
+                    const int i0 = x0 - 1, i1 = x0 + t.w;
+                    auto take = [&](size_t k, int i, int j) {
+                        GhostOp op = P.fill[ring0 + k];
+                        op.dst = (i - i0) + (j - (y0 - 1)) * (t.w + 2);
                         P.tile_fill.push_back(op);
-                    }
+                    };
+                    if (x0 == 0)
+                        for (int j = j0; j <= j1; ++j) take((size_t)j, -1, j);
+                    if (i1 == nx)
+                        for (int j = j0; j <= j1; ++j) take((size_t)ny + j, nx, j);
+                    if (y0 == 0)
+                        for (int i = i0; i <= i1; ++i) take((size_t)2 * ny + (i + 1), i, -1);
+                    if (y0 + t.h == ny)
+                        for (int i = i0; i <= i1; ++i) take((size_t)2 * ny + (nx + 2) + (i + 1), i, ny);
                     t.fill1 = (int)P.tile_fill.size();
                     P.tiles.push_back(t);
                 }
