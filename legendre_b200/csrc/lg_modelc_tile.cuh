@@ -153,9 +153,28 @@ __device__ __forceinline__ void flush_edges(T* __restrict__ out, const SlabLayou
 // The new phi and u of a cell from its drift (kphi, ku): the Euler-Maruyama
 // update (MODE 0) or a RungeKutta4 stage (MODE 1 to 3); e0/e1 index the cell's
 // phi/u entries in any arena of the state's layout.
+//
+// RkCell: the other operands of a cell's stage, loaded before the drift they
+// are added to is known.
+template <class T>
+struct RkCell {
+    T y0, y1, a0, a1;
+};
+template <class T, int MODE>
+__device__ __forceinline__ void rk_load(const RkArgs<T>& rk, int64_t e0, int64_t e1, RkCell<T>& c) {
+    if constexpr (MODE >= 2) {
+        c.a0 = rk.acc[e0];
+        c.a1 = rk.acc[e1];
+    }
+    if constexpr (MODE == 2) {
+        c.y0 = __ldg(rk.y + e0);
+        c.y1 = __ldg(rk.y + e1);
+    }
+}
 template <class T, class Ops, bool NOISE, int MODE>
-__device__ __forceinline__ void cell_update(const RkArgs<T>& rk, T dt, T scale_amp, T nval, T kphi, T ku, T p, T uc,
-                                            int64_t e0, int64_t e1, bool ok, T& phin, T& un) {
+__device__ __forceinline__ void cell_update(const RkArgs<T>& rk, const RkCell<T>& rc, T dt, T scale_amp, T nval,
+                                            T kphi, T ku, T p, T uc, int64_t e0, int64_t e1, bool ok, T& phin,
+                                            T& un) {
     if constexpr (MODE == 0) {
         phin = Ops::axpy(dt, kphi, p);
         if (NOISE) phin = Ops::add_noise(phin, scale_amp, nval);
@@ -168,14 +187,14 @@ __device__ __forceinline__ void cell_update(const RkArgs<T>& rk, T dt, T scale_a
             rk.acc[e1] = uc + rk.s * ku;
         }
     } else {
-        phin = un = T(0);  // cells that store nothing read nothing either
-        if (!ok) return;
-        const T a0 = rk.acc[e0] + rk.s * kphi, a1 = rk.acc[e1] + rk.s * ku;
+        const T a0 = rc.a0 + rk.s * kphi, a1 = rc.a1 + rk.s * ku;
         if constexpr (MODE == 2) {
-            phin = rk.y[e0] + rk.c * kphi;
-            un = rk.y[e1] + rk.c * ku;
-            rk.acc[e0] = a0;
-            rk.acc[e1] = a1;
+            phin = rc.y0 + rk.c * kphi;
+            un = rc.y1 + rk.c * ku;
+            if (ok) {
+                rk.acc[e0] = a0;
+                rk.acc[e1] = a1;
+            }
         } else {
             phin = a0;
             un = a1;
@@ -240,6 +259,8 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
         ul = __ldg(uu + off - 1);
         ur = __ldg(uu + off + 1);
     }
+    RkCell<T> rc{};
+    if (live) rk_load<T, MODE>(rk, (po - out) + off, (uo - out) + off, rc);
     T nval = T(0);
     if (NOISE) nval = Ops::noise(splitmix64(block_key ^ (uint64_t)(col + j * n0)));
     if constexpr (ORIENT) {
@@ -274,7 +295,7 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
         T kphi, ku;
         Ops::ocell(m, jr, jl, jt, jbot, B.b, B.c - B.a, C.b - A.b, c0, s0, UB, ul, ur, UC, UA, kphi, ku);
         T phin, un;
-        cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off,
+        cell_update<T, Ops, NOISE, MODE>(rk, rc, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off,
                                          (uo - out) + off, ok, phin, un);
         store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L, nb, eh);
         jb = jt;
@@ -291,7 +312,7 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
     T kphi, ku;
     Ops::cell(m, fr, fl, jt, jb, B.b, B.c - B.a, C.b - A.b, UB, ul, ur, UC, UA, kphi, ku);
     T phin, un;
-    cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off, (uo - out) + off,
+    cell_update<T, Ops, NOISE, MODE>(rk, rc, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off, (uo - out) + off,
                                      ok, phin, un);
     store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L, nb, eh);
     jb = jt;
@@ -500,6 +521,9 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             asm volatile("prefetch.global.L1 [%0];" ::"l"(uu + off + p3));
             asm volatile("prefetch.global.L1 [%0];" ::"l"(uu + off + p4));
         }
+        RkCell<T> rc0{}, rc1{};
+        rk_load<T, MODE>(rk, (po - out) + off, (uo - out) + off, rc0);
+        rk_load<T, MODE>(rk, (po - out) + off + sy, (uo - out) + off + sy, rc1);
         const T ul0 = __ldg(uu + off - 1), ur0 = __ldg(uu + off + 1);
         const T ul1 = __ldg(uu + off + sy - 1), ur1 = __ldg(uu + off + sy + 1);
         T c0 = T(0), s0 = T(0), c1 = T(0), s1 = T(0);  // multi-grain: frames of rows j and j+1
@@ -528,9 +552,9 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
         const bool own0 = j >= rs, own1 = j + 1 >= rs;
         auto update = [&](T kphi0, T ku0, T kphi1, T ku1) {
             const int64_t e0 = (po - out) + off, e1 = (uo - out) + off;
-            cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nv0, kphi0, ku0, B.b, UB, e0, e1, ok && own0, phin0,
+            cell_update<T, Ops, NOISE, MODE>(rk, rc0, dt, scale_amp, nv0, kphi0, ku0, B.b, UB, e0, e1, ok && own0, phin0,
                                              un0);
-            cell_update<T, Ops, NOISE, MODE>(rk, dt, scale_amp, nv1, kphi1, ku1, C.b, UC, e0 + sy, e1 + sy,
+            cell_update<T, Ops, NOISE, MODE>(rk, rc1, dt, scale_amp, nv1, kphi1, ku1, C.b, UC, e0 + sy, e1 + sy,
                                              ok && own1, phin1, un1);
         };
         if constexpr (MODE >= 2) {  // the stage's other operands of the next pass
