@@ -91,49 +91,80 @@ struct RkArgs {
     T c, s;
 };
 
-// Ghost images of a strip's x-edge cells (the block's columns 0 and n0 - 1)
-// for the rows of one unit: lane k holds row r0 + k's phi and u of the left
-// (l0, l1) and right (r0, r1) edge cells, gathered by shuffles as the rows
-// are stepped and written once at the unit's end (rows 0 and n1 - 1, whose
-// images include y ghosts and corners, are pushed in full as they go).
+// Ghost images of a strip's x-edge cells (the block's columns 0 and n0 - 1;
+// rows 0 and n1 - 1, whose images include y ghosts and corners, are pushed in
+// full).  FP64: the lane that owns an edge cell keeps the address of its image
+// in the unit's first row -- the neighbour's ghost column, or this block's own
+// at a mirror boundary -- and stores there as it stores the cell.  FP32: the
+// images are gathered by shuffles, lane k holding those of row r0 + k (l0, l1:
+// phi and u of the left edge cell, q0, q1: of the right one), and written once
+// at the unit's end.  (The FP64 gather is 32 shuffles and selects a pass:
+// 2002^2 in blocks of 91 x 77 without noise 61 -> 58 us a step with stores as
+// the rows go, 10080^2 1357 -> 1327, but FP32 4096^2 in blocks of 256^2 143 ->
+// 147.)
 template <class T>
-struct EdgeHold {
-    T l0, l1, r0, r1;
+struct EdgeImages {
+    static constexpr bool kGather = sizeof(T) == 4;
+    T* p;  // this lane's image in row r0; null: not an edge cell
+    T l0, l1, q0, q1;
+    __device__ __forceinline__ EdgeImages(T* __restrict__ out, const SlabLayout& L, const Nbr2& nb, int n0, int r0,
+                                          int col)
+        : p(nullptr), l0(T(0)), l1(T(0)), q0(T(0)), q1(T(0)) {
+        if constexpr (!kGather) {
+            if (col == 0)
+                p = out + slab_base(L, nb.l >= 0 ? nb.l : nb.b, 0) + (nb.l >= 0 ? n0 + 1 : 0);
+            else if (col == n0 - 1)
+                p = out + slab_base(L, nb.r >= 0 ? nb.r : nb.b, 0) + (nb.r >= 0 ? 0 : n0 + 1);
+            if (p) p += (int64_t)(r0 + 1) * L.gdim[0];
+        }
+    }
+    // one row of a strip on a block's x edge (the whole warp calls)
+    __device__ __forceinline__ void row(T phin, T un, bool ok, bool live, int k, int lane, int last_lane, int sy,
+                                        int64_t slab_stride) {
+        if constexpr (kGather) {
+            const T a0 = __shfl_sync(0xffffffffu, phin, 0), a1 = __shfl_sync(0xffffffffu, un, 0);
+            const T b0 = __shfl_sync(0xffffffffu, phin, last_lane), b1 = __shfl_sync(0xffffffffu, un, last_lane);
+            if (live && lane == (k & 31)) {
+                l0 = a0;
+                l1 = a1;
+                q0 = b0;
+                q1 = b1;
+            }
+        } else if (ok && p) {
+            T* const q = p + (int64_t)k * sy;
+            q[0] = phin;
+            q[slab_stride] = un;
+        }
+    }
 };
 
-// store the cell, and take care of its ghost images (see EdgeHold)
+// store the cell, and take care of its ghost images (see EdgeImages;
+// one-column blocks push every row in full)
 template <class T>
 __device__ __forceinline__ void store_cell(T* __restrict__ out, T* __restrict__ po, T* __restrict__ uo, int off,
                                            T phin, T un, bool ok, bool live, bool edge_x, int j, int r0, int n0,
-                                           int n1, int col, int lane, int last_lane, const SlabLayout& L,
-                                           const Nbr2& nb, EdgeHold<T>& eh) {
+                                           int n1, int col, int lane, int last_lane, int sy, const SlabLayout& L,
+                                           const Nbr2& nb, EdgeImages<T>& eh) {
     if (ok) {
         po[off] = phin;
         uo[off] = un;
     }
-    if (j == 0 || j == n1 - 1) {  // warp-uniform
+    if (j == 0 || j == n1 - 1 || (!EdgeImages<T>::kGather && n0 == 1)) {  // warp-uniform
         if (ok) {
             push_ghosts_2d_g1(out, L, 0, nb, n0, n1, col, j, phin);
             push_ghosts_2d_g1(out, L, 1, nb, n0, n1, col, j, un);
         }
-    } else if (edge_x) {  // warp-uniform: warps on a block's x edge collect their edge cells
-        const T l0 = __shfl_sync(0xffffffffu, phin, 0), l1 = __shfl_sync(0xffffffffu, un, 0);
-        const T rr0 = __shfl_sync(0xffffffffu, phin, last_lane), rr1 = __shfl_sync(0xffffffffu, un, last_lane);
-        if (live && lane == ((j - r0) & 31)) {
-            eh.l0 = l0;
-            eh.l1 = l1;
-            eh.r0 = rr0;
-            eh.r1 = rr1;
-        }
+    } else if (edge_x) {  // warp-uniform
+        eh.row(phin, un, ok, live, j - r0, lane, last_lane, sy, L.slab_stride);
     }
 }
 
 // the collected x-edge images of a unit's rows (r0 .. r1-1, not 0 or n1-1):
 // the left edge's into the left neighbour's ghost column n0 (or this block's
-// mirror ghost column -1), the right edge's likewise (push_ghosts_2d_g1)
+// mirror ghost column -1), the right edge's likewise (push_ghosts_2d_g1); FP32 only
 template <class T>
 __device__ __forceinline__ void flush_edges(T* __restrict__ out, const SlabLayout& L, const Nbr2& nb, int n0, int n1,
-                                            int r0, int r1, int lane, bool left, bool right, const EdgeHold<T>& eh,
+                                            int r0, int r1, int lane, bool left, bool right, const EdgeImages<T>& eh,
                                             int rs = -1) {
     const int r = r0 + lane;
     if (r >= r1 || r < rs || r == 0 || r == n1 - 1) return;  // rows below rs: another unit's
@@ -145,8 +176,8 @@ __device__ __forceinline__ void flush_edges(T* __restrict__ out, const SlabLayou
     }
     if (right) {
         const int tb = nb.r >= 0 ? nb.r : nb.b, ci = nb.r >= 0 ? -1 : n0;
-        out[slab_base(L, tb, 0) + (ci + 1) + row] = eh.r0;
-        out[slab_base(L, tb, 1) + (ci + 1) + row] = eh.r1;
+        out[slab_base(L, tb, 0) + (ci + 1) + row] = eh.q0;
+        out[slab_base(L, tb, 1) + (ci + 1) + row] = eh.q1;
     }
 }
 
@@ -235,8 +266,8 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
                                           uint64_t block_key, T bnd, const Row3<T>& A, const Row3<T>& B,
                                           const Row3<T>& C, Row3<T>& P, T UA, T UB, T UC, T& UP, T& jb, T dt,
                                           T scale_amp, const T* __restrict__ trig_b, int64_t ncells, T& cprev,
-                                          T& sprev, T& cnext, T& snext, const RkArgs<T>& rk, EdgeHold<T>& eh,
-                                          int rs) {
+                                          T& sprev, T& cnext, T& snext, const RkArgs<T>& rk,
+                                          EdgeImages<T>& eh, int rs) {
     const int sy = NX > 0 ? NX + 2 : g.L.gdim[0];
     // lanes past the block's last column (valid false) run the same code on
     // a clamped column and only skip the stores: no branch splits the face,
@@ -297,7 +328,7 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
         T phin, un;
         cell_update<T, Ops, NOISE, MODE>(rk, rc, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off,
                                          (uo - out) + off, ok, phin, un);
-        store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L, nb, eh);
+        store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, sy, g.L, nb, eh);
         jb = jt;
         cprev = c0;
         sprev = s0;
@@ -314,7 +345,7 @@ __device__ __forceinline__ void strip_row(const typename Ops::Params& m, const T
     T phin, un;
     cell_update<T, Ops, NOISE, MODE>(rk, rc, dt, scale_amp, nval, kphi, ku, B.b, UB, (po - out) + off, (uo - out) + off,
                                      ok, phin, un);
-    store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L, nb, eh);
+    store_cell(out, po, uo, off, phin, un, ok, live, edge_x, j, r0, n0, n1, col, lane, last_lane, sy, g.L, nb, eh);
     jb = jt;
 }
 
@@ -389,7 +420,7 @@ __device__ __forceinline__ void strip_unit(const typename Ops::Params& m, uint64
         jb = Ops::oyface(m, cpv, spv, T(0.25) * (w[1].c - w[1].a + w[0].c - w[0].a), w[1].b - w[0].b);
     }
 
-    EdgeHold<T> eh{T(0), T(0), T(0), T(0)};
+    EdgeImages<T> eh(out, g.L, nb, n0, r0, col);
 #define LG_ROW(J, Q)                                                                                            \
     strip_row<T, Ops, NOISE, NX, FULL, PF, TAIL, ORIENT, MODE>(m, g, J, r0, r1, lane, col, valid, last_lane, n0, n1, off, ph, uu, out, po,  \
                                        uo, nb, edge_x, block_key, bnd, w[(Q) % NB], w[((Q) + 1) % NB],          \
@@ -421,7 +452,8 @@ __device__ __forceinline__ void strip_unit(const typename Ops::Params& m, uint64
         }
     }
 #undef LG_ROW
-    if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
+    if constexpr (EdgeImages<T>::kGather)
+        if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
 }
 
 // The paired form of one work unit (Euler-Maruyama, axis-aligned, units of
@@ -499,7 +531,7 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
     } else {
         jb = Ops::yface(m, B.b - A.b, B.c - B.a, A.c, A.a);
     }
-    EdgeHold<T> eh{T(0), T(0), T(0), T(0)};
+    EdgeImages<T> eh(out, g.L, nb, n0, r0, col);
 #pragma unroll 1
     for (int j = r0; j < r1; j += 2) {
         // the four rows of this pass (j-1 .. j+2 <= n1) from L1, and an L1
@@ -645,14 +677,15 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             }
             update(kphi0, ku0, kphi1, ku1);
         }
-        store_cell(out, po, uo, off, phin0, un0, ok && own0, own0, edge_x, j, r0, n0, n1, col, lane, last_lane, g.L,
-                   nb, eh);
+        store_cell(out, po, uo, off, phin0, un0, ok && own0, own0, edge_x, j, r0, n0, n1, col, lane, last_lane, sy,
+                   g.L, nb, eh);
         store_cell(out, po, uo, off + sy, phin1, un1, ok && own1, own1, edge_x, j + 1, r0, n0, n1, col, lane,
-                   last_lane, g.L, nb, eh);
+                   last_lane, sy, g.L, nb, eh);
         jb = jt1;
         off += 2 * sy;
     }
-    if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
+    if constexpr (EdgeImages<T>::kGather)
+        if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
 }
 
 // strip, row chunk and block of a work unit
