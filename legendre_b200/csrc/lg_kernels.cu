@@ -96,9 +96,10 @@ __device__ __forceinline__ void push_ghost_images(T* __restrict__ arena, const C
 // the other rows one entry a thread.
 //
 // Bound: DRAM and L2 sectors (an x ghost costs a sector read and one written
-// for its 8 bytes).  All index arithmetic is 32 bit, two divisions an entry;
-// with 64-bit divisions in every dimension the fill of 32,768 blocks of 16^3
-// took 1650 us, as long as three and a half heat steps.
+// for its 8 bytes) and the latency of a copy, so each thread has four in
+// flight: the fill of 32,768 blocks of 16^3 takes 470 us, one entry at a time
+// 660.  All index arithmetic is 32 bit, two divisions an entry; with 64-bit
+// divisions in every dimension it took 1650 us, three and a half heat steps.
 template <int D, class T>
 __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, CartTopo topo, SlabLayout L,
                                                         int field) {
@@ -135,38 +136,55 @@ __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, C
             if (mirror[e][step >> 1]) return step == 0 ? -1 - i : 2 * n - 1 - i;
             return step == 0 ? n + i : i - n;
         };
-        auto copy = [&](int x, int y, int z) {
+        // element offsets of ghost entry (x, y, z) in its slab and of its
+        // source in the arena
+        auto place = [&](int x, int y, int z, int64_t& to, int64_t& from) {
             int sx, sy = 1, sz = 1;
             const int mx = map(0, x, n0, sx);
             const int my = D > 1 ? map(1, y, n1, sy) : 0;
             const int mz = D > 2 ? map(2, z, n2, sz) : 0;
             const int code = sx + (D > 1 ? 3 * sy : 0) + (D > 2 ? 9 * sz : 0);
-            const int64_t to = (x + g) + (int64_t)G0 * ((y + gy) + (int64_t)G1 * (z + gz));
-            const int64_t from = (mx + g) + (int64_t)G0 * ((my + gy) + (int64_t)G1 * (mz + gz));
-            slab[to] = arena[src_base[code] + from];
+            to = (x + g) + (int64_t)G0 * ((y + gy) + (int64_t)G1 * (z + gz));
+            from = src_base[code] + (mx + g) + (int64_t)G0 * ((my + gy) + (int64_t)G1 * (mz + gz));
         };
-        // x ghosts of the interior rows: 2 g entries a row
-        const unsigned rows = (unsigned)n1 * n2, per = 2u * g;
-        for (unsigned k = first; k < rows * per; k += stride) {
-            const unsigned row = k / per, i = k - row * per;
-            const unsigned z = row / n1, y = row - z * n1;
-            copy((int)i < g ? (int)i - g : n0 + (int)i - g, (int)y, (int)z);
-        }
-        if (D > 1) {  // rows with y outside, z inside
-            const unsigned strip = 2u * g * G0;
-            for (unsigned k = first; k < strip * n2; k += stride) {
+        // the entries in one sequence: x ghosts of the interior rows (2 g a
+        // row), rows with y outside and z inside, planes with z outside
+        const unsigned per = 2u * g, xs = (unsigned)n1 * n2 * per;
+        const unsigned strip = D > 1 ? 2u * g * G0 : 1, ys = D > 1 ? xs + strip * n2 : xs;
+        const unsigned plane = D > 2 ? (unsigned)G0 * G1 : 1, all = D > 2 ? ys + plane * 2u * g : ys;
+        auto entry = [&](unsigned k, int64_t& to, int64_t& from) {
+            if (k < xs) {
+                const unsigned row = k / per, i = k - row * per;
+                const unsigned z = row / n1, y = row - z * n1;
+                place((int)i < g ? (int)i - g : n0 + (int)i - g, (int)y, (int)z, to, from);
+            } else if (D > 1 && k < ys) {
+                k -= xs;
                 const unsigned z = k / strip, q = k - z * strip;
                 const unsigned r = q / G0, x = q - r * G0;
-                copy((int)x - g, (int)r < g ? (int)r - g : n1 + (int)r - g, (int)z);
-            }
-        }
-        if (D > 2) {  // planes with z outside
-            const unsigned plane = (unsigned)G0 * G1;
-            for (unsigned k = first; k < plane * 2u * g; k += stride) {
+                place((int)x - g, (int)r < g ? (int)r - g : n1 + (int)r - g, (int)z, to, from);
+            } else if (D > 2) {
+                k -= ys;
                 const unsigned p = k / plane, q = k - p * plane;
                 const unsigned r = q / G0, x = q - r * G0;
-                copy((int)x - g, (int)r - g, (int)p < g ? (int)p - g : n2 + (int)p - g);
+                place((int)x - g, (int)r - g, (int)p < g ? (int)p - g : n2 + (int)p - g, to, from);
             }
+        };
+        constexpr int U = 4;  // entries in flight a thread
+        for (unsigned k = first; k < all; k += U * stride) {
+            int64_t to[U];
+            T v[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const unsigned e = k + u * stride;
+                if (e < all) {
+                    int64_t from = 0;
+                    entry(e, to[u], from);
+                    v[u] = arena[from];
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+                if (k + u * stride < all) slab[to[u]] = v[u];
         }
     }
 }
