@@ -561,6 +561,12 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
         T c0 = T(0), s0 = T(0), c1 = T(0), s1 = T(0);  // multi-grain: frames of rows j and j+1
         if constexpr (ORIENT) {
             const int64_t ci = (int64_t)j * n0 + ccol;
+            const int64_t p2 = ci + (int64_t)(min(j + 2, n1 - 1) - j) * n0;  // the next pass's frames
+            const int64_t p3 = ci + (int64_t)(min(j + 3, n1 - 1) - j) * n0;
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p2));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p2));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p3));
+            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p3));
             c0 = __ldg(trig_b + ci);
             s0 = __ldg(trig_b + ncells + ci);
             c1 = __ldg(trig_b + ci + n0);
