@@ -31,7 +31,7 @@ __device__ __forceinline__ float rcp_approx(float x) {
 
 struct OpsFast32 {
     using Params = Fast32;
-    static constexpr bool kFarPass = true;  // the paired rows test for the far field first (quarter, *_far)
+    static constexpr bool kGuarded = false;  // no range test to leave out: SAFE means nothing here
 
     static __device__ __forceinline__ void aniso(float dx, float dy, float a_bar, float a1pe, float two_ae,
                                                  float tol, float& a, float& inv) {
@@ -43,6 +43,7 @@ struct OpsFast32 {
         a = flat ? a_bar : a1pe - two_ae * (dx2 * dy2) * inv;
         inv = flat ? 0.0f : inv;
     }
+    template <bool SAFE = false>
     static __device__ __forceinline__ float xface(const Fast32& m, float dn, float d1, float c, float e) {
         const float dt = 0.25f * ((d1 + c) - e);
         float a, inv;
@@ -50,6 +51,7 @@ struct OpsFast32 {
         const float da = -m.f_a12 * dn * dt * (dn * dn - dt * dt) * inv;
         return a * (a * dn - da * dt);
     }
+    template <bool SAFE = false>
     static __device__ __forceinline__ float yface(const Fast32& m, float dn, float d1, float c, float e) {
         const float dt = 0.25f * ((d1 + c) - e);
         float a, inv;
@@ -108,15 +110,42 @@ struct OpsFast32 {
     // with the flat selects taken.
     static __device__ __forceinline__ float quarter(float d1, float c, float e) { return 0.25f * ((d1 + c) - e); }
     static __device__ __forceinline__ int far_key(const Fast32& m) { return m.far_key; }
+    static __device__ __forceinline__ int safe_key(const Fast32&) { return 0x7fffffff; }
     static __device__ __forceinline__ int face_key(float dx, float dy) { return order_key(dx * dx + dy * dy); }
     static __device__ __forceinline__ int center_key(float cdx, float cdy) {
         return quarter_key(cdx * cdx + cdy * cdy);
     }
     static __device__ __forceinline__ float xface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ float yface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
-    static __device__ __forceinline__ void cell_far(const Fast32& m, float jr, float jl, float jt, float jb, float p,
-                                                    float uc, float ul, float ur, float up, float um, float& kphi,
-                                                    float& ku) {
+    // the cell's drift; nothing is left open
+    struct Cell {
+        float kphi, ku;
+    };
+    template <bool SAFE = false>
+    static __device__ __forceinline__ Cell cell_open(const Fast32& m, float jr, float jl, float jt, float jb, float p,
+                                                     float cdx, float cdy, float uc, float ul, float ur, float up,
+                                                     float um) {
+        Cell o;
+        cell(m, jr, jl, jt, jb, p, cdx, cdy, uc, ul, ur, up, um, o.kphi, o.ku);
+        return o;
+    }
+    static __device__ __forceinline__ Cell ocell_open(const Fast32& m, float jr, float jl, float jt, float jb, float p,
+                                                      float cdx, float cdy, float c0, float s0, float uc, float ul,
+                                                      float ur, float up, float um) {
+        Cell o;
+        ocell(m, jr, jl, jt, jb, p, cdx, cdy, c0, s0, uc, ul, ur, up, um, o.kphi, o.ku);
+        return o;
+    }
+    static __device__ __forceinline__ void close2(const Fast32&, const Cell& o0, const Cell& o1, float& kphi0,
+                                                  float& ku0, float& kphi1, float& ku1) {
+        kphi0 = o0.kphi;
+        ku0 = o0.ku;
+        kphi1 = o1.kphi;
+        ku1 = o1.ku;
+    }
+    static __device__ __forceinline__ Cell cell_far(const Fast32& m, float jr, float jl, float jt, float jb, float p,
+                                                    float uc, float ul, float ur, float up, float um) {
+        float kphi, ku;
         const float flux = ((jr - jl) + (jt - jb)) * m.inv_h2_flux;
         const float g_prime = p * p * p - p;
         const float one_m_p2 = 1.0f - p * p;
@@ -124,6 +153,7 @@ struct OpsFast32 {
         kphi = ((flux - g_prime) - m.lambda * uc * p_prime) * rcp_approx(m.c_a_bar * m.c_a_bar);
         const float lap = ((ur + ul) - 2.0f * uc) * m.ih0 + ((up + um) - 2.0f * uc) * m.ih1;
         ku = lap * m.d_thermal + 0.5f * kphi;
+        return {kphi, ku};
     }
     static __device__ __forceinline__ float axpy(float dt, float k, float x) { return x + dt * k; }
     static __device__ __forceinline__ float noise(uint64_t key) { return normal_fast32(key); }

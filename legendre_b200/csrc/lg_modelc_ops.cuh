@@ -16,7 +16,8 @@ template <class T>
 struct MC {
     T lambda, d_thermal, a_bar, eps_prime, tol, f_a_bar, f_eps_prime, f_a12, f_tol, inv_h2_flux, ih0, ih1;
     T c_far, inv_c_far;  // a_bar * a_bar, the far-field mobility divisor, and RN(1 / c_far)
-    int far_key;         // largest gradient key that is flat for certain (see gradient_key)
+    int far_key;         // largest gradient key that is flat for certain (far_key_of)
+    int safe_key;        // gradient keys below it are in the reciprocals' range (safe_key_of)
 };
 
 // The high half of a non-negative double, or the bits of a non-negative
@@ -53,6 +54,15 @@ inline int far_key_of(T tol) {
     return order_key(s) - 1;
 }
 
+// Passes whose gradients' keys are all below it divide by nothing outside
+// recip_rn's range: |grad|^2 < 2^450, and a non-flat |grad|^4 is above the
+// tolerances, which must not be tiny themselves (else no pass is safe).
+template <class T>
+inline int safe_key_of(T f_tol, T tol) {
+    const bool tiny = !(f_tol >= T(0x1p-100) && tol >= T(0x1p-100));
+    return tiny ? -0x7fffffff - 1 : order_key((T)(sizeof(T) == 8 ? 0x1p450 : 0x1p60));
+}
+
 template <class T>
 inline MC<T> to_mc(const ModelCDev& m) {
     MC<T> r;
@@ -71,6 +81,7 @@ inline MC<T> to_mc(const ModelCDev& m) {
     r.c_far = r.a_bar * r.a_bar;
     r.inv_c_far = T(1) / r.c_far;
     r.far_key = far_key_of(std::min(r.f_tol, r.tol));
+    r.safe_key = safe_key_of(r.f_tol, r.tol);
     return r;
 }
 
@@ -103,9 +114,12 @@ __device__ __forceinline__ bool recip_range(double c) {
 // the division itself, out of line: for operands outside the ranges above
 static __device__ __noinline__ double ieee_quotient(double x, double c) { return x / c; }
 
-// the two ratios of a non-flat face: n1 / c and n2 / c, the IEEE quotients
+// the two ratios of a non-flat face: n1 / c and n2 / c, the IEEE quotients.
+// SAFE: the caller knows c to be in recip_rn's range; the test and the call
+// behind it cost the FP64 step 7 %.
+template <bool SAFE>
 __device__ __forceinline__ void ratios(double n1, double n2, double c, double& q1, double& q2) {
-    if (recip_range(c)) {
+    if (SAFE || recip_range(c)) {
         const double y = recip_rn(c);
         q1 = quotient_rn(n1, c, y);
         q2 = quotient_rn(n2, c, y);
@@ -114,18 +128,21 @@ __device__ __forceinline__ void ratios(double n1, double n2, double c, double& q
         q2 = ieee_quotient(n2, c);
     }
 }
+template <bool SAFE>
 __device__ __forceinline__ void ratios(float n1, float n2, float c, float& q1, float& q2) {
     q1 = n1 / c;
     q2 = n2 / c;
 }
+template <bool SAFE>
 __device__ __forceinline__ double ratio(double n, double c) {
-    return recip_range(c) ? quotient_rn(n, c, recip_rn(c)) : ieee_quotient(n, c);
+    return SAFE || recip_range(c) ? quotient_rn(n, c, recip_rn(c)) : ieee_quotient(n, c);
 }
+template <bool SAFE>
 __device__ __forceinline__ float ratio(float n, float c) { return n / c; }
 
 // KarmaRappelFlux::face (finite_volume.rs:129-142); its two quotients share
 // one reciprocal
-template <class T>
+template <bool SAFE = false, class T>
 __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da) {
     T dx2 = dx * dx;
     T dy2 = dy * dy;
@@ -136,7 +153,7 @@ __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da)
         da = T(0);
     } else {
         T q1, q2;
-        ratios(m.f_eps_prime * (dx2 * dx2 + dy2 * dy2), -(m.f_a12) * dx * dy * (dx2 - dy2), mag2, q1, q2);
+        ratios<SAFE>(m.f_eps_prime * (dx2 * dx2 + dy2 * dy2), -(m.f_a12) * dx * dy * (dx2 - dy2), mag2, q1, q2);
         a = m.f_a_bar * (T(1) + q1);
         da = q2;
     }
@@ -144,14 +161,14 @@ __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da)
 
 // ModelC::center_anisotropy (phasefield.rs:159-175) from the half
 // differences dx = 0.5 (p(i+1) - p(i-1)), dy likewise.
-template <class T>
+template <bool SAFE = false, class T>
 __device__ __forceinline__ T center_anisotropy(const MC<T>& m, T dx, T dy) {
     T dx2 = dx * dx;
     T dy2 = dy * dy;
     T sum = dx2 + dy2;
     T mag2 = sum * sum;
     if (mag2 <= m.tol) return m.a_bar;
-    return m.a_bar * (T(1) + ratio(m.eps_prime * (dx2 * dx2 + dy2 * dy2), mag2));
+    return m.a_bar * (T(1) + ratio<SAFE>(m.eps_prime * (dx2 * dx2 + dy2 * dy2), mag2));
 }
 
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
@@ -159,30 +176,32 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(
 
 __device__ __forceinline__ double normal_t(uint64_t key, double) { return standard_normal(key); }
 
-// x / c_far, the IEEE quotient, for the far-field cells (a = a_bar).  For
-// double operands whose quotient neither underflows nor overflows, the
-// quotient q = RN(x y) by the correctly rounded reciprocal y = RN(1/c)
-// followed by one correction with the exact residual r = x - c q (an fma),
-// RN(q + r y), is the correctly rounded x / c (Markstein's theorem; the
-// same bits as the division, checked against it on 3.8e9 operands over
-// 600 divisors, half of them next to rounding midpoints).  Zeros are x y
-// (their sign kept); tiny and huge x take the division.
-__device__ __forceinline__ double div_far(double x, double c, double y) {
-    const double q = x * y;
-    const double qc = fma(fma(-q, c, x), y, q);
-    const unsigned ex = (unsigned)__double2hiint(x) << 1;  // exponent above the sign
-    const bool in = ex - 0x07e00000u < 0xf0200000u;  // 2^-960 <= |x| < 2^961
-    if (!in && x != 0.0) return ieee_quotient(x, c);
-    return in ? qc : q;  // +-0 / c = +-0 = +-0 y (y > 0)
+// The mobility quotients x0 / c0 and x1 / c1 of two cells (c = a^2, y = RN(1 /
+// c)): the IEEE quotients for |x| >= 2^-960 (below, where the residual
+// underflows, within an ulp; a zero's sign is not kept).  Where one comes out
+// infinite or NaN -- an overflow, a divisor of zero, such an operand -- both are
+// divided again.
+__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7fffffff) >= 0x7ff00000; }
+__device__ __forceinline__ double mobility(double x, double c, double y) {
+    const double k = quotient_rn(x, c, y);
+    return not_finite(k) ? ieee_quotient(x, c) : k;
 }
-__device__ __forceinline__ float div_far(float x, float c, float) { return x / c; }
-// x / c, the IEEE quotient, for the mobility divisor c = a^2 of one cell
-__device__ __forceinline__ double div_cell(double x, double c) {
-    const unsigned ex = (unsigned)__double2hiint(x) << 1;  // exponent above the sign
-    if (ex - 0x0f600000u < 0xe1000000u && recip_range(c)) return quotient_rn(x, c, recip_rn(c));
-    return ieee_quotient(x, c);
+__device__ __forceinline__ void mobility2(double x0, double c0, double y0, double x1, double c1, double y1, double& k0,
+                                          double& k1) {
+    k0 = quotient_rn(x0, c0, y0);
+    k1 = quotient_rn(x1, c1, y1);
+    if (max(__double2hiint(k0) & 0x7fffffff, __double2hiint(k1) & 0x7fffffff) >= 0x7ff00000) {
+        k0 = ieee_quotient(x0, c0);
+        k1 = ieee_quotient(x1, c1);
+    }
 }
-__device__ __forceinline__ float div_cell(float x, float c) { return x / c; }
+__device__ __forceinline__ double mobility_recip(double c) { return recip_rn(c); }
+__device__ __forceinline__ float mobility(float x, float c, float) { return x / c; }
+__device__ __forceinline__ void mobility2(float x0, float c0, float, float x1, float c1, float, float& k0, float& k1) {
+    k0 = x0 / c0;
+    k1 = x1 / c1;
+}
+__device__ __forceinline__ float mobility_recip(float) { return 0.0f; }
 __device__ __forceinline__ float normal_t(uint64_t key, float) { return standard_normal_f32(key); }
 
 // The exact FP64 arithmetic policy of the step kernels: face fluxes from
@@ -193,20 +212,22 @@ __device__ __forceinline__ float normal_t(uint64_t key, float) { return standard
 template <class T>
 struct OpsExact {
     using Params = MC<T>;
-    static constexpr bool kFarPass = true;  // the paired rows test for the far field first (quarter, *_far)
+    static constexpr bool kGuarded = true;   // SAFE forms leave a range test out
 
     // x face: KarmaRappelFlux::face(derx, dery) and j = a (a derx - da dery)
+    template <bool SAFE = false>
     static __device__ __forceinline__ T xface(const MC<T>& m, T dn, T d1, T c, T e) {
         const T dt = T(0.25) * (d1 + c - e);
         T a, da;
-        kr_face(m, dn, dt, a, da);
+        kr_face<SAFE>(m, dn, dt, a, da);
         return a * (a * dn - da * dt);
     }
     // y face: face(derx, dery) with derx transverse, j = a (a dery + da derx)
+    template <bool SAFE = false>
     static __device__ __forceinline__ T yface(const MC<T>& m, T dn, T d1, T c, T e) {
         const T dt = T(0.25) * (d1 + c - e);
         T a, da;
-        kr_face(m, dt, dn, a, da);
+        kr_face<SAFE>(m, dt, dn, a, da);
         return a * (a * dn + da * dt);
     }
     // The far-field forms: the face fluxes and the cell update with the
@@ -217,38 +238,61 @@ struct OpsExact {
     // face in the reference's rounding.
     static __device__ __forceinline__ T quarter(T d1, T c, T e) { return T(0.25) * (d1 + c - e); }
     static __device__ __forceinline__ int far_key(const MC<T>& m) { return m.far_key; }
+    static __device__ __forceinline__ int safe_key(const MC<T>& m) { return m.safe_key; }
     static __device__ __forceinline__ int face_key(T dx, T dy) { return order_key(fma_t(dx, dx, dy * dy)); }
     // from the whole differences p(i+1) - p(i-1)
     static __device__ __forceinline__ int center_key(T cdx, T cdy) { return quarter_key(fma_t(cdx, cdx, cdy * cdy)); }
     static __device__ __forceinline__ T xface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ T yface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
-    static __device__ __forceinline__ void cell_far(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T uc, T ul, T ur,
-                                                    T up, T um, T& kphi, T& ku) {
+
+    // A cell's dphi/dt = num / c and du/dt = fma(lap, d_thermal, 0.5 dphi/dt),
+    // the quotient left open so that the two cells of a pass share its test
+    struct Cell {
+        T num, c, y, lap;
+    };
+    static __device__ __forceinline__ void open(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T uc, T ul, T ur, T up,
+                                                T um, Cell& o) {
         const T flux = (jr - jl + jt - jb) * m.inv_h2_flux;
         const T g_prime = fma_t(p * p, p, -p);
         const T one_m_p2 = fma_t(p, -p, T(1));
         const T p_prime = one_m_p2 * one_m_p2;
-        kphi = div_far(fma_t(m.lambda * uc, -p_prime, flux - g_prime), m.c_far, m.inv_c_far);
+        o.num = fma_t(m.lambda * uc, -p_prime, flux - g_prime);
         T acc = T(0);
         acc += ((ur - (uc + uc)) + ul) * m.ih0;
         acc += ((up - (uc + uc)) + um) * m.ih1;
-        ku = fma_t(acc, m.d_thermal, T(0.5) * kphi);
+        o.lap = acc;
+    }
+    static __device__ __forceinline__ Cell cell_far(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T uc, T ul, T ur,
+                                                    T up, T um) {
+        Cell o;
+        open(m, jr, jl, jt, jb, p, uc, ul, ur, up, um, o);
+        o.c = m.c_far;
+        o.y = m.inv_c_far;
+        return o;
+    }
+    template <bool SAFE = false>
+    static __device__ __forceinline__ Cell cell_open(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T cdx, T cdy, T uc,
+                                                     T ul, T ur, T up, T um) {
+        Cell o;
+        open(m, jr, jl, jt, jb, p, uc, ul, ur, up, um, o);
+        const T a = center_anisotropy<SAFE>(m, T(0.5) * cdx, T(0.5) * cdy);
+        o.c = a * a;
+        o.y = mobility_recip(o.c);
+        return o;
+    }
+    static __device__ __forceinline__ void close(const MC<T>& m, const Cell& o, T& kphi, T& ku) {
+        kphi = mobility(o.num, o.c, o.y);
+        ku = fma_t(o.lap, m.d_thermal, T(0.5) * kphi);
+    }
+    static __device__ __forceinline__ void close2(const MC<T>& m, const Cell& o0, const Cell& o1, T& kphi0, T& ku0,
+                                                  T& kphi1, T& ku1) {
+        mobility2(o0.num, o0.c, o0.y, o1.num, o1.c, o1.y, kphi0, kphi1);
+        ku0 = fma_t(o0.lap, m.d_thermal, T(0.5) * kphi0);
+        ku1 = fma_t(o1.lap, m.d_thermal, T(0.5) * kphi1);
     }
     static __device__ __forceinline__ void cell(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T cdx, T cdy, T uc,
                                                 T ul, T ur, T up, T um, T& kphi, T& ku) {
-        const T flux = (jr - jl + jt - jb) * m.inv_h2_flux;
-        const T g_prime = fma_t(p * p, p, -p);
-        const T one_m_p2 = fma_t(p, -p, T(1));
-        const T p_prime = one_m_p2 * one_m_p2;
-        const T a = center_anisotropy(m, T(0.5) * cdx, T(0.5) * cdy);
-        const T num = fma_t(m.lambda * uc, -p_prime, flux - g_prime);
-        // a == a_bar: the divisor a a is c_far (whichever branch of the
-        // anisotropy gave it)
-        kphi = a == m.a_bar ? div_far(num, m.c_far, m.inv_c_far) : div_cell(num, a * a);
-        T acc = T(0);
-        acc += ((ur - (uc + uc)) + ul) * m.ih0;
-        acc += ((up - (uc + uc)) + um) * m.ih1;
-        ku = fma_t(acc, m.d_thermal, T(0.5) * kphi);
+        close(m, cell_open(m, jr, jl, jt, jb, p, cdx, cdy, uc, ul, ur, up, um), kphi, ku);
     }
     // Multi-grain faces and cell (finite_volume.rs:196-234, phasefield.rs:
     // 378-392): a face's anisotropy in the crystal frame (c0, s0) = (cos, sin)
@@ -266,21 +310,20 @@ struct OpsExact {
         kr_face(m, c0 * derx + s0 * dery, c0 * dery - s0 * derx, a, da);
         return a * (a * dery + da * derx);
     }
-    static __device__ __forceinline__ void ocell(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T cdx, T cdy, T c0, T s0,
-                                                 T uc, T ul, T ur, T up, T um, T& kphi, T& ku) {
-        const T flux = (jr - jl + jt - jb) * m.inv_h2_flux;
-        const T g_prime = fma_t(p * p, p, -p);
-        const T one_m_p2 = fma_t(p, -p, T(1));
-        const T p_prime = one_m_p2 * one_m_p2;
+    static __device__ __forceinline__ Cell ocell_open(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T cdx, T cdy, T c0,
+                                                      T s0, T uc, T ul, T ur, T up, T um) {
+        Cell o;
+        open(m, jr, jl, jt, jb, p, uc, ul, ur, up, um, o);
         const T dx = T(0.5) * cdx, dy = T(0.5) * cdy;
         T a, da;
         kr_face(m, c0 * dx + s0 * dy, c0 * dy - s0 * dx, a, da);
-        const T num = fma_t(m.lambda * uc, -p_prime, flux - g_prime);
-        kphi = a == m.f_a_bar ? div_far(num, m.c_far, m.inv_c_far) : div_cell(num, a * a);
-        T acc = T(0);
-        acc += ((ur - (uc + uc)) + ul) * m.ih0;
-        acc += ((up - (uc + uc)) + um) * m.ih1;
-        ku = fma_t(acc, m.d_thermal, T(0.5) * kphi);
+        o.c = a * a;
+        o.y = mobility_recip(o.c);
+        return o;
+    }
+    static __device__ __forceinline__ void ocell(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T cdx, T cdy, T c0, T s0,
+                                                 T uc, T ul, T ur, T up, T um, T& kphi, T& ku) {
+        close(m, ocell_open(m, jr, jl, jt, jb, p, cdx, cdy, c0, s0, uc, ul, ur, up, um), kphi, ku);
     }
     static __device__ __forceinline__ T axpy(T dt, T k, T x) { return x + dt * k; }
     static __device__ __forceinline__ T noise(uint64_t key) { return normal_t(key, T(0)); }

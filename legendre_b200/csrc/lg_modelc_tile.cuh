@@ -43,6 +43,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 
 #include "lg_common.cuh"
 #include "lg_kernels.h"
@@ -632,55 +633,62 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
                 jbot0 = Ops::oyface(m, c0, s0, q * (B.c - B.a + A.c - A.a), B.b - A.b);
             if (!(same_bits(c0, c1) && same_bits(s0, s1)))
                 jbot1 = Ops::oyface(m, c1, s1, q * (C.c - C.a + B.c - B.a), C.b - B.b);
+            const auto o0 = Ops::ocell_open(m, jr0, jl0, jt0, jbot0, B.b, B.c - B.a, C.b - A.b, c0, s0, UB, ul0,
+                                            ur0, UC, UA);
+            const auto o1 = Ops::ocell_open(m, jr1, jl1, jt1, jbot1, C.b, C.c - C.a, D.b - B.b, c1, s1, UC, ul1,
+                                            ur1, UD, UB);
             T kphi0, ku0, kphi1, ku1;
-            Ops::ocell(m, jr0, jl0, jt0, jbot0, B.b, B.c - B.a, C.b - A.b, c0, s0, UB, ul0, ur0, UC, UA, kphi0, ku0);
-            Ops::ocell(m, jr1, jl1, jt1, jbot1, C.b, C.c - C.a, D.b - B.b, c1, s1, UC, ul1, ur1, UD, UB, kphi1, ku1);
+            Ops::close2(m, o0, o1, kphi0, ku0, kphi1, ku1);
             update(kphi0, ku0, kphi1, ku1);
             cprev = c1;
             sprev = s1;
         } else {
-            T fl0, jt0, fl1;
-            T kphi0, ku0, kphi1, ku1;
-            bool far = false;
-            if constexpr (Ops::kFarPass) {
-                // the four faces' and two centres' gradients; where all are
-                // flat for certain across the warp (the far field) the pass
-                // runs without branches, with the general path's values
-                const T xn0 = B.b - B.a, xt0 = Ops::quarter(C.b - A.b, C.a, A.a);
-                const T yn0 = C.b - B.b, yt0 = Ops::quarter(C.c - C.a, B.c, B.a);
-                const T xn1 = C.b - C.a, xt1 = Ops::quarter(D.b - B.b, D.a, B.a);
-                const T yn1 = D.b - C.b, yt1 = Ops::quarter(D.c - D.a, C.c, C.a);
-                const int key = max(max(max(Ops::face_key(xn0, xt0), Ops::face_key(yt0, yn0)),
-                                        max(Ops::face_key(xn1, xt1), Ops::face_key(yt1, yn1))),
-                                    max(Ops::center_key(B.c - B.a, C.b - A.b), Ops::center_key(C.c - C.a, D.b - B.b)));
-                far = __all_sync(kFull, key <= Ops::far_key(m));
-                if (far) {
-                    fl0 = Ops::xface_far(m, xn0);
-                    jt0 = Ops::yface_far(m, yn0);
-                    fl1 = Ops::xface_far(m, xn1);
-                    jt1 = Ops::yface_far(m, yn1);
-                    T fr0 = __shfl_down_sync(kFull, fl0, 1), fr1 = __shfl_down_sync(kFull, fl1, 1);
-                    if (lane == last_lane) {
-                        fr0 = fb0;
-                        fr1 = fb1;
-                    }
-                    Ops::cell_far(m, fr0, fl0, jt0, jb, B.b, UB, ul0, ur0, UC, UA, kphi0, ku0);
-                    Ops::cell_far(m, fr1, fl1, jt1, jt0, C.b, UC, ul1, ur1, UD, UB, kphi1, ku1);
-                }
-            }
-            if (!far) {
-                fl0 = Ops::xface(m, B.b - B.a, C.b - A.b, C.a, A.a);
-                jt0 = Ops::yface(m, C.b - B.b, C.c - C.a, B.c, B.a);
-                fl1 = Ops::xface(m, C.b - C.a, D.b - B.b, D.a, B.a);
-                jt1 = Ops::yface(m, D.b - C.b, D.c - D.a, C.c, C.a);
-                T fr0 = __shfl_down_sync(kFull, fl0, 1), fr1 = __shfl_down_sync(kFull, fl1, 1);
+            // the four faces' and two centres' gradients; where all are flat
+            // for certain across the warp (the far field) the pass runs without
+            // branches, with the general path's values; elsewhere the general
+            // path leaves its range tests out where the gradients allow it
+            const T xn0 = B.b - B.a, xt0 = Ops::quarter(C.b - A.b, C.a, A.a);
+            const T yn0 = C.b - B.b, yt0 = Ops::quarter(C.c - C.a, B.c, B.a);
+            const T xn1 = C.b - C.a, xt1 = Ops::quarter(D.b - B.b, D.a, B.a);
+            const T yn1 = D.b - C.b, yt1 = Ops::quarter(D.c - D.a, C.c, C.a);
+            const int key = max(max(max(Ops::face_key(xn0, xt0), Ops::face_key(yt0, yn0)),
+                                    max(Ops::face_key(xn1, xt1), Ops::face_key(yt1, yn1))),
+                                max(Ops::center_key(B.c - B.a, C.b - A.b), Ops::center_key(C.c - C.a, D.b - B.b)));
+            typename Ops::Cell o0, o1;
+            auto right_faces = [&](T fl0, T fl1, T& fr0, T& fr1) {
+                fr0 = __shfl_down_sync(kFull, fl0, 1);
+                fr1 = __shfl_down_sync(kFull, fl1, 1);
                 if (lane == last_lane) {
                     fr0 = fb0;
                     fr1 = fb1;
                 }
-                Ops::cell(m, fr0, fl0, jt0, jb, B.b, B.c - B.a, C.b - A.b, UB, ul0, ur0, UC, UA, kphi0, ku0);
-                Ops::cell(m, fr1, fl1, jt1, jt0, C.b, C.c - C.a, D.b - B.b, UC, ul1, ur1, UD, UB, kphi1, ku1);
+            };
+            auto general = [&](auto safe) {
+                constexpr bool S = decltype(safe)::value;
+                const T fl0 = Ops::template xface<S>(m, B.b - B.a, C.b - A.b, C.a, A.a);
+                const T jt0 = Ops::template yface<S>(m, C.b - B.b, C.c - C.a, B.c, B.a);
+                const T fl1 = Ops::template xface<S>(m, C.b - C.a, D.b - B.b, D.a, B.a);
+                jt1 = Ops::template yface<S>(m, D.b - C.b, D.c - D.a, C.c, C.a);
+                T fr0, fr1;
+                right_faces(fl0, fl1, fr0, fr1);
+                o0 = Ops::template cell_open<S>(m, fr0, fl0, jt0, jb, B.b, B.c - B.a, C.b - A.b, UB, ul0, ur0, UC, UA);
+                o1 = Ops::template cell_open<S>(m, fr1, fl1, jt1, jt0, C.b, C.c - C.a, D.b - B.b, UC, ul1, ur1, UD,
+                                                UB);
+            };
+            if (__all_sync(kFull, key <= Ops::far_key(m))) {
+                const T fl0 = Ops::xface_far(m, xn0), jt0 = Ops::yface_far(m, yn0), fl1 = Ops::xface_far(m, xn1);
+                jt1 = Ops::yface_far(m, yn1);
+                T fr0, fr1;
+                right_faces(fl0, fl1, fr0, fr1);
+                o0 = Ops::cell_far(m, fr0, fl0, jt0, jb, B.b, UB, ul0, ur0, UC, UA);
+                o1 = Ops::cell_far(m, fr1, fl1, jt1, jt0, C.b, UC, ul1, ur1, UD, UB);
+            } else if (!Ops::kGuarded || __all_sync(kFull, key < Ops::safe_key(m))) {
+                general(std::true_type{});
+            } else {
+                general(std::false_type{});
             }
+            T kphi0, ku0, kphi1, ku1;
+            Ops::close2(m, o0, o1, kphi0, ku0, kphi1, ku1);
             update(kphi0, ku0, kphi1, ku1);
         }
         store_cell(out, po, uo, off, phin0, un0, ok && own0, own0, edge_x, j, r0, n0, n1, col, lane, last_lane, sy,
