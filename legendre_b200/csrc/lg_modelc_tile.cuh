@@ -457,9 +457,9 @@ __device__ __forceinline__ void strip_unit(const typename Ops::Params& m, uint64
         if (edge_x) flush_edges(out, g.L, nb, n0, n1, r0, r1, lane, col - lane == 0, cr == n0 - 1, eh, rs);
 }
 
-// The paired form of one work unit (Euler-Maruyama, axis-aligned, units of
-// an even number of rows): each pass of the row loop steps rows j and j+1
-// together, so every lane carries two independent cells -- four face fluxes,
+// The paired form of one work unit (an Euler-Maruyama step or an RK4 stage,
+// axis-aligned or multi-grain; units of an even number of rows): each pass of
+// the row loop steps rows j and j+1 together, so every lane carries two independent cells -- four face fluxes,
 // two Gaussians, two cell updates -- whose dependency chains the scheduler
 // interleaves; the y face between the two rows is computed once.  Each pass
 // reads its four phi and u rows j-1 .. j+2 from L1, where the previous pass
