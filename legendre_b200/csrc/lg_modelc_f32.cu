@@ -20,7 +20,7 @@ struct Fast32 {
     float lambda, d_thermal, inv_h2_flux, ih0, ih1;
     float f_a_bar, f_a1pe, f_2ae, f_a12, f_tol;  // flux: a, a(1+e'), 2 a e', a12, tol
     float c_a_bar, c_a1pe, c_2ae, c_tol;         // cell-centred anisotropy
-    int far_key;
+    unsigned far_face, far_center;               // gradient keys below them are flat (far_below)
 };
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -109,12 +109,11 @@ struct OpsFast32 {
     // reciprocal the general form takes.  Same values as the general forms
     // with the flat selects taken.
     static __device__ __forceinline__ float quarter(float d1, float c, float e) { return 0.25f * ((d1 + c) - e); }
-    static __device__ __forceinline__ int far_key(const Fast32& m) { return m.far_key; }
-    static __device__ __forceinline__ int safe_key(const Fast32&) { return 0x7fffffff; }
-    static __device__ __forceinline__ int face_key(float dx, float dy) { return order_key(dx * dx + dy * dy); }
-    static __device__ __forceinline__ int center_key(float cdx, float cdy) {
-        return quarter_key(cdx * cdx + cdy * cdy);
+    static __device__ __forceinline__ bool far(const Fast32& m, unsigned faces, unsigned centers) {
+        return faces < m.far_face && centers < m.far_center;
     }
+    static __device__ __forceinline__ bool safe(const Fast32&, unsigned, unsigned) { return true; }
+    static __device__ __forceinline__ unsigned key(float dx, float dy) { return order_key(dx * dx + dy * dy); }
     static __device__ __forceinline__ float xface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ float yface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     // the cell's drift; nothing is left open
@@ -193,7 +192,8 @@ Fast32 fast32_of(const ModelCDev& m) {
     f.c_a1pe = (float)(m.a_bar * (1.0 + m.eps_prime));
     f.c_2ae = (float)(2.0 * m.a_bar * m.eps_prime);
     f.c_tol = (float)m.tol;
-    f.far_key = far_key_of(std::min(f.f_tol, f.c_tol));
+    f.far_face = far_below(f.f_tol, false);
+    f.far_center = far_below(f.c_tol, true);
     return f;
 }
 }  // namespace

@@ -6,6 +6,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <limits>
 
 #include "lg_common.cuh"
 #include "lg_kernels.h"
@@ -16,51 +17,54 @@ template <class T>
 struct MC {
     T lambda, d_thermal, a_bar, eps_prime, tol, f_a_bar, f_eps_prime, f_a12, f_tol, inv_h2_flux, ih0, ih1;
     T c_far, inv_c_far;  // a_bar * a_bar, the far-field mobility divisor, and RN(1 / c_far)
-    int far_key;         // largest gradient key that is flat for certain (far_key_of)
-    int safe_key;        // gradient keys below it are in the reciprocals' range (safe_key_of)
+    unsigned far_face;    // face and centre keys below these are flat for certain (far_below)
+    unsigned far_center;
+    unsigned safe_below;  // gradient keys below it are in the reciprocals' range (safe_below_of)
 };
 
 // The high half of a non-negative double, or the bits of a non-negative
-// float, ordered as the values are.
-__host__ __device__ __forceinline__ int order_key(double s) {
+// float: an unsigned number ordered as the values are, with every NaN above
+// them all (one whose sign bit is set, as an invalid operation leaves it in a
+// double, too).
+__host__ __device__ __forceinline__ unsigned order_key(double s) {
 #ifdef __CUDA_ARCH__
-    return __double2hiint(s);
+    return (unsigned)__double2hiint(s);
 #else
-    int64_t b;
+    uint64_t b;
     memcpy(&b, &s, sizeof b);
-    return (int)(b >> 32);
+    return (unsigned)(b >> 32);
 #endif
 }
-__host__ __device__ __forceinline__ int order_key(float s) {
+__host__ __device__ __forceinline__ unsigned order_key(float s) {
 #ifdef __CUDA_ARCH__
-    return __float_as_int(s);
+    return __float_as_uint(s);
 #else
-    int b;
+    unsigned b;
     memcpy(&b, &s, sizeof b);
     return b;
 #endif
 }
-// a key of s / 4
-__device__ __forceinline__ int quarter_key(double s) { return order_key(s) - (2 << 20); }
-__device__ __forceinline__ int quarter_key(float s) { return order_key(s) - (2 << 23); }
 
 // The far field (|grad|^4 <= tol, in the reference's rounding) decided
-// without its rounding: every |grad|^2 whose key is at most far_key_of(tol)
-// is below sqrt(tol) by more than any rounding of the sum and its square.
+// without its rounding: every |grad|^2 whose key is below the limit is below
+// sqrt(tol) by more than any rounding of the sum and its square.  A limit of
+// zero: none.  far_center is the limit for 4 |grad|^2, the sum of the whole
+// differences' squares; no limit reaches the keys of infinity and NaN.
 template <class T>
-inline int far_key_of(T tol) {
-    if (!(tol > T(0))) return -0x7fffffff - 1;
+inline unsigned far_below(T tol, bool center) {
+    if (!(tol > T(0))) return 0;
     const T s = std::sqrt(tol) * (T(1) - (sizeof(T) == 8 ? T(0x1p-40) : T(0x1p-20)));
-    return order_key(s) - 1;
+    const unsigned two = 2u << (sizeof(T) == 8 ? 20 : 23);  // two binades
+    return std::min(order_key(s) + (center ? two : 0u), order_key(std::numeric_limits<T>::infinity()));
 }
 
-// Passes whose gradients' keys are all below it divide by nothing outside
+// Passes whose gradients' keys are all below safe_below divide by nothing outside
 // recip_rn's range: |grad|^2 < 2^450, and a non-flat |grad|^4 is above the
 // tolerances, which must not be tiny themselves (else no pass is safe).
 template <class T>
-inline int safe_key_of(T f_tol, T tol) {
+inline unsigned safe_below_of(T f_tol, T tol) {
     const bool tiny = !(f_tol >= T(0x1p-100) && tol >= T(0x1p-100));
-    return tiny ? -0x7fffffff - 1 : order_key((T)(sizeof(T) == 8 ? 0x1p450 : 0x1p60));
+    return tiny ? 0 : order_key((T)(sizeof(T) == 8 ? 0x1p450 : 0x1p60));
 }
 
 template <class T>
@@ -80,8 +84,9 @@ inline MC<T> to_mc(const ModelCDev& m) {
     r.ih1 = (T)m.inv_h2[1];
     r.c_far = r.a_bar * r.a_bar;
     r.inv_c_far = T(1) / r.c_far;
-    r.far_key = far_key_of(std::min(r.f_tol, r.tol));
-    r.safe_key = safe_key_of(r.f_tol, r.tol);
+    r.far_face = far_below(r.f_tol, false);
+    r.far_center = far_below(r.tol, true);
+    r.safe_below = safe_below_of(r.f_tol, r.tol);
     return r;
 }
 
@@ -233,15 +238,18 @@ struct OpsExact {
     // The far-field forms: the face fluxes and the cell update with the
     // anisotropy branches decided (kr_face and center_anisotropy both flat):
     // a = f_a_bar, da = 0, and a dn - 0 dt is a dn (the transverse difference
-    // is finite where the test holds).  The test is conservative (far_key_of):
+    // is finite where the test holds).  The test is conservative (far_below):
     // a pass that fails it takes the general path, whose branches decide each
     // face in the reference's rounding.
     static __device__ __forceinline__ T quarter(T d1, T c, T e) { return T(0.25) * (d1 + c - e); }
-    static __device__ __forceinline__ int far_key(const MC<T>& m) { return m.far_key; }
-    static __device__ __forceinline__ int safe_key(const MC<T>& m) { return m.safe_key; }
-    static __device__ __forceinline__ int face_key(T dx, T dy) { return order_key(fma_t(dx, dx, dy * dy)); }
-    // from the whole differences p(i+1) - p(i-1)
-    static __device__ __forceinline__ int center_key(T cdx, T cdy) { return quarter_key(fma_t(cdx, cdx, cdy * cdy)); }
+    static __device__ __forceinline__ bool far(const MC<T>& m, unsigned faces, unsigned centers) {
+        return faces < m.far_face && centers < m.far_center;
+    }
+    static __device__ __forceinline__ bool safe(const MC<T>& m, unsigned faces, unsigned centers) {
+        return max(faces, centers) < m.safe_below;
+    }
+    // of a face's differences, and of a centre's whole ones (p(i+1) - p(i-1))
+    static __device__ __forceinline__ unsigned key(T dx, T dy) { return order_key(fma_t(dx, dx, dy * dy)); }
     static __device__ __forceinline__ T xface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ T yface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
 

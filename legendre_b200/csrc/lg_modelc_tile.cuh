@@ -651,9 +651,9 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             const T yn0 = C.b - B.b, yt0 = Ops::quarter(C.c - C.a, B.c, B.a);
             const T xn1 = C.b - C.a, xt1 = Ops::quarter(D.b - B.b, D.a, B.a);
             const T yn1 = D.b - C.b, yt1 = Ops::quarter(D.c - D.a, C.c, C.a);
-            const int key = max(max(max(Ops::face_key(xn0, xt0), Ops::face_key(yt0, yn0)),
-                                    max(Ops::face_key(xn1, xt1), Ops::face_key(yt1, yn1))),
-                                max(Ops::center_key(B.c - B.a, C.b - A.b), Ops::center_key(C.c - C.a, D.b - B.b)));
+            const unsigned faces =
+                max(max(Ops::key(xn0, xt0), Ops::key(yt0, yn0)), max(Ops::key(xn1, xt1), Ops::key(yt1, yn1)));
+            const unsigned centers = max(Ops::key(B.c - B.a, C.b - A.b), Ops::key(C.c - C.a, D.b - B.b));
             typename Ops::Cell o0, o1;
             auto right_faces = [&](T fl0, T fl1, T& fr0, T& fr1) {
                 fr0 = __shfl_down_sync(kFull, fl0, 1);
@@ -675,14 +675,14 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
                 o1 = Ops::template cell_open<S>(m, fr1, fl1, jt1, jt0, C.b, C.c - C.a, D.b - B.b, UC, ul1, ur1, UD,
                                                 UB);
             };
-            if (__all_sync(kFull, key <= Ops::far_key(m))) {
+            if (__all_sync(kFull, Ops::far(m, faces, centers))) {
                 const T fl0 = Ops::xface_far(m, xn0), jt0 = Ops::yface_far(m, yn0), fl1 = Ops::xface_far(m, xn1);
                 jt1 = Ops::yface_far(m, yn1);
                 T fr0, fr1;
                 right_faces(fl0, fl1, fr0, fr1);
                 o0 = Ops::cell_far(m, fr0, fl0, jt0, jb, B.b, UB, ul0, ur0, UC, UA);
                 o1 = Ops::cell_far(m, fr1, fl1, jt1, jt0, C.b, UC, ul1, ur1, UD, UB);
-            } else if (!Ops::kGuarded || __all_sync(kFull, key < Ops::safe_key(m))) {
+            } else if (!Ops::kGuarded || __all_sync(kFull, Ops::safe(m, faces, centers))) {
                 general(std::true_type{});
             } else {
                 general(std::false_type{});
