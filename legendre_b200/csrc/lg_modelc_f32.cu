@@ -112,7 +112,8 @@ struct OpsFast32 {
     static __device__ __forceinline__ bool far(const Fast32& m, unsigned faces, unsigned centers) {
         return faces < m.far_face && centers < m.far_center;
     }
-    static __device__ __forceinline__ bool safe(const Fast32&, unsigned, unsigned) { return true; }
+    static __device__ __forceinline__ bool safe(const Fast32&, unsigned, unsigned, float, float) { return true; }
+    static __device__ __forceinline__ bool divides(const Fast32&) { return false; }
     static __device__ __forceinline__ unsigned key(float dx, float dy) { return order_key(dx * dx + dy * dy); }
     static __device__ __forceinline__ float xface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
     static __device__ __forceinline__ float yface_far(const Fast32& m, float dn) { return m.f_a_bar * (m.f_a_bar * dn); }
@@ -120,6 +121,7 @@ struct OpsFast32 {
     struct Cell {
         float kphi, ku;
     };
+    static __device__ __forceinline__ void divide(Cell&) {}
     template <bool SAFE = false>
     static __device__ __forceinline__ Cell cell_open(const Fast32& m, float jr, float jl, float jt, float jb, float p,
                                                      float cdx, float cdy, float uc, float ul, float ur, float up,
@@ -135,7 +137,7 @@ struct OpsFast32 {
         ocell(m, jr, jl, jt, jb, p, cdx, cdy, c0, s0, uc, ul, ur, up, um, o.kphi, o.ku);
         return o;
     }
-    static __device__ __forceinline__ void close2(const Fast32&, const Cell& o0, const Cell& o1, float& kphi0,
+    static __device__ __forceinline__ void close2(const Fast32&, const Cell& o0, const Cell& o1, bool, float& kphi0,
                                                   float& ku0, float& kphi1, float& ku1) {
         kphi0 = o0.kphi;
         ku0 = o0.ku;

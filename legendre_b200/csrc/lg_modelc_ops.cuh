@@ -10,6 +10,7 @@
 
 #include "lg_common.cuh"
 #include "lg_kernels.h"
+#include "lg_quotient.cuh"
 
 namespace lg {
 
@@ -19,22 +20,15 @@ struct MC {
     T c_far, inv_c_far;  // a_bar * a_bar, the far-field mobility divisor, and RN(1 / c_far)
     unsigned far_face;    // face and centre keys below these are flat for certain (far_below)
     unsigned far_center;
-    unsigned safe_below;  // gradient keys below it are in the reciprocals' range (safe_below_of)
+    unsigned quotient_span;  // of the divisors that the faces' quotients take (quotient_span_of)
+    unsigned safe_below;     // gradient keys below it are in that range (safe_below_of)
 };
 
 // The high half of a non-negative double, or the bits of a non-negative
 // float: an unsigned number ordered as the values are, with every NaN above
 // them all (one whose sign bit is set, as an invalid operation leaves it in a
 // double, too).
-__host__ __device__ __forceinline__ unsigned order_key(double s) {
-#ifdef __CUDA_ARCH__
-    return (unsigned)__double2hiint(s);
-#else
-    uint64_t b;
-    memcpy(&b, &s, sizeof b);
-    return (unsigned)(b >> 32);
-#endif
-}
+__host__ __device__ __forceinline__ unsigned order_key(double s) { return high_word(s); }
 __host__ __device__ __forceinline__ unsigned order_key(float s) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(s);
@@ -58,13 +52,28 @@ inline unsigned far_below(T tol, bool center) {
     return std::min(order_key(s) + (center ? two : 0u), order_key(std::numeric_limits<T>::infinity()));
 }
 
-// Passes whose gradients' keys are all below safe_below divide by nothing outside
-// recip_rn's range: |grad|^2 < 2^450, and a non-flat |grad|^4 is above the
+// The quotients take the shared reciprocal for parameters as ordinary as
+// these: a face's divisor |grad|^4 in [2^-900, 2^60) then keeps its first
+// numerator e' (dx^4 + dy^4), at least half e' |grad|^4, and both quotients in
+// quotient_rn's range, so that only a tiny second numerator is left to test,
+// and the mobility's divisor a^2 stays below 2^60.  Others divide.
+template <class T>
+inline unsigned quotient_span_of(const MC<T>& m) {
+    auto within = [](T e, T most) { return std::fabs(e) >= T(0x1p-50) && std::fabs(e) <= most; };
+    auto none_or = [&](T e, T most) { return e == T(0) || within(e, most); };
+    return none_or(m.eps_prime, T(0x1p10)) && none_or(m.f_eps_prime, T(0x1p10)) && none_or(m.f_a12, T(0x1p40)) &&
+                   within(m.a_bar, T(0x1p18)) && within(m.f_a_bar, T(0x1p18))
+               ? kQuotientSpan
+               : 0;
+}
+
+// Passes whose gradients' keys are all below safe_below have every divisor in
+// that range: |grad|^2 < 2^29, and a non-flat |grad|^4 is above the
 // tolerances, which must not be tiny themselves (else no pass is safe).
 template <class T>
-inline unsigned safe_below_of(T f_tol, T tol) {
-    const bool tiny = !(f_tol >= T(0x1p-100) && tol >= T(0x1p-100));
-    return tiny ? 0 : order_key((T)(sizeof(T) == 8 ? 0x1p450 : 0x1p60));
+inline unsigned safe_below_of(const MC<T>& m) {
+    const bool tiny = !(m.f_tol >= T(0x1p-100) && m.tol >= T(0x1p-100));
+    return tiny || m.quotient_span == 0 ? 0 : order_key(T(0x1p29));
 }
 
 template <class T>
@@ -84,47 +93,31 @@ inline MC<T> to_mc(const ModelCDev& m) {
     r.ih1 = (T)m.inv_h2[1];
     r.c_far = r.a_bar * r.a_bar;
     r.inv_c_far = T(1) / r.c_far;
-    r.far_face = far_below(r.f_tol, false);
-    r.far_center = far_below(r.tol, true);
-    r.safe_below = safe_below_of(r.f_tol, r.tol);
+    r.quotient_span = quotient_span_of(r);
+    // the far forms drop a zero's addition to a face flux, whose sign shows in
+    // no result for these parameters
+    const bool far = r.quotient_span && r.f_a_bar > T(0.5) && r.d_thermal >= T(0);
+    r.far_face = far ? far_below(r.f_tol, false) : 0;
+    r.far_center = far ? far_below(r.tol, true) : 0;
+    r.safe_below = safe_below_of(r);
     return r;
 }
 
-// RN(1 / c) for 2^-900 <= |c| <= 2^900: the hardware's approximation (better
-// than 2^-19), one cubic step, y (1 + e + e^2) with e = 1 - c y, and one
-// correction with the exact residual, which gives the correctly rounded
-// reciprocal unless every bit of c's mantissa is set (Markstein, IBM J. Res.
-// Dev. 34, 1990).
-__device__ __forceinline__ double recip_rn(double c) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(c));
-    double e = fma(-c, y, 1.0);
-    e = fma(e, e, e);
-    y = fma(y, e, y);
-    return fma(y, fma(-c, y, 1.0), y);
-}
-// RN(x / c) with y = RN(1 / c): the quotient RN(x y) corrected with its exact
-// residual (the same theorem).  Against the division on 1.2e9 operands, near
-// rounding midpoints and with mantissas of all ones among them: no mismatch.
-// x = 0 gives a zero (its sign is not kept).
-__device__ __forceinline__ double quotient_rn(double x, double c, double y) {
-    const double q = x * y;
-    return fma(fma(-q, c, x), y, q);
-}
-// 2^-900 <= |c| < 2^900, where recip_rn holds
-__device__ __forceinline__ bool recip_range(double c) {
-    return (unsigned)(__double2hiint(c) & 0x7fffffff) - 0x07b00000u < 0x70800000u;
-}
-
-// the division itself, out of line: for operands outside the ranges above
+// the division itself, out of line: for operands outside the ranges of the
+// shared reciprocal
 static __device__ __noinline__ double ieee_quotient(double x, double c) { return x / c; }
 
-// the two ratios of a non-flat face: n1 / c and n2 / c, the IEEE quotients.
-// SAFE: the caller knows c to be in recip_rn's range; the test and the call
-// behind it cost the FP64 step 7 %.
-template <bool SAFE>
-__device__ __forceinline__ void ratios(double n1, double n2, double c, double& q1, double& q2) {
-    if (SAFE || recip_range(c)) {
+// The two ratios of a non-flat face, n1 / c and n2 / c: the IEEE quotients.
+// SAFE: the caller knows them to be in range (OpsExact::safe); the tests
+// here and the calls behind them cost the FP64 step 7 %.
+template <bool SAFE, class T>
+__device__ __forceinline__ void ratios(const MC<T>&, float n1, float n2, float c, float& q1, float& q2) {
+    q1 = n1 / c;
+    q2 = n2 / c;
+}
+template <bool SAFE, class T>
+__device__ __forceinline__ void ratios(const MC<T>& m, double n1, double n2, double c, double& q1, double& q2) {
+    if (SAFE || (recip_range(c, m.quotient_span) && fabs(n2) >= kQuotientLow)) {
         const double y = recip_rn(c);
         q1 = quotient_rn(n1, c, y);
         q2 = quotient_rn(n2, c, y);
@@ -133,17 +126,12 @@ __device__ __forceinline__ void ratios(double n1, double n2, double c, double& q
         q2 = ieee_quotient(n2, c);
     }
 }
-template <bool SAFE>
-__device__ __forceinline__ void ratios(float n1, float n2, float c, float& q1, float& q2) {
-    q1 = n1 / c;
-    q2 = n2 / c;
+template <bool SAFE, class T>
+__device__ __forceinline__ float ratio(const MC<T>&, float n, float c) { return n / c; }
+template <bool SAFE, class T>
+__device__ __forceinline__ double ratio(const MC<T>& m, double n, double c) {
+    return SAFE || recip_range(c, m.quotient_span) ? quotient_rn(n, c, recip_rn(c)) : ieee_quotient(n, c);
 }
-template <bool SAFE>
-__device__ __forceinline__ double ratio(double n, double c) {
-    return SAFE || recip_range(c) ? quotient_rn(n, c, recip_rn(c)) : ieee_quotient(n, c);
-}
-template <bool SAFE>
-__device__ __forceinline__ float ratio(float n, float c) { return n / c; }
 
 // KarmaRappelFlux::face (finite_volume.rs:129-142); its two quotients share
 // one reciprocal
@@ -158,7 +146,7 @@ __device__ __forceinline__ void kr_face(const MC<T>& m, T dx, T dy, T& a, T& da)
         da = T(0);
     } else {
         T q1, q2;
-        ratios<SAFE>(m.f_eps_prime * (dx2 * dx2 + dy2 * dy2), -(m.f_a12) * dx * dy * (dx2 - dy2), mag2, q1, q2);
+        ratios<SAFE>(m, m.f_eps_prime * (dx2 * dx2 + dy2 * dy2), -(m.f_a12) * dx * dy * (dx2 - dy2), mag2, q1, q2);
         a = m.f_a_bar * (T(1) + q1);
         da = q2;
     }
@@ -173,7 +161,7 @@ __device__ __forceinline__ T center_anisotropy(const MC<T>& m, T dx, T dy) {
     T sum = dx2 + dy2;
     T mag2 = sum * sum;
     if (mag2 <= m.tol) return m.a_bar;
-    return m.a_bar * (T(1) + ratio<SAFE>(m.eps_prime * (dx2 * dx2 + dy2 * dy2), mag2));
+    return m.a_bar * (T(1) + ratio<SAFE>(m, m.eps_prime * (dx2 * dx2 + dy2 * dy2), mag2));
 }
 
 __device__ __forceinline__ double fma_t(double a, double b, double c) { return fma(a, b, c); }
@@ -181,28 +169,26 @@ __device__ __forceinline__ float fma_t(float a, float b, float c) { return fmaf(
 
 __device__ __forceinline__ double normal_t(uint64_t key, double) { return standard_normal(key); }
 
-// The mobility quotients x0 / c0 and x1 / c1 of two cells (c = a^2, y = RN(1 /
-// c)): the IEEE quotients for |x| >= 2^-960 (below, where the residual
-// underflows, within an ulp; a zero's sign is not kept).  Where one comes out
-// infinite or NaN -- an overflow, a divisor of zero, such an operand -- both are
-// divided again.
-__device__ __forceinline__ bool not_finite(double x) { return (__double2hiint(x) & 0x7fffffff) >= 0x7ff00000; }
-__device__ __forceinline__ double mobility(double x, double c, double y) {
+// The mobility quotient x / c of a cell, c = a^2 and y = RN(1 / c)
+__device__ __forceinline__ double mobility(const MC<double>& m, double x, double c, double y) {
     const double k = quotient_rn(x, c, y);
-    return not_finite(k) ? ieee_quotient(x, c) : k;
+    return quotient_suspect(x, k, x, k) | (m.quotient_span == 0) ? ieee_quotient(x, c) : k;
 }
-__device__ __forceinline__ void mobility2(double x0, double c0, double y0, double x1, double c1, double y1, double& k0,
-                                          double& k1) {
+// of two cells, which share a test (the tests for tiny numerators cost 10080^2
+// 0.6 % and 512^2 0.8 %); `divide`: their divisors may be out of range
+__device__ __forceinline__ void mobility2(double x0, double c0, double y0, double x1, double c1, double y1, bool divide,
+                                          double& k0, double& k1) {
     k0 = quotient_rn(x0, c0, y0);
     k1 = quotient_rn(x1, c1, y1);
-    if (max(__double2hiint(k0) & 0x7fffffff, __double2hiint(k1) & 0x7fffffff) >= 0x7ff00000) {
+    if (divide | quotient_suspect(x0, k0, x1, k1)) {
         k0 = ieee_quotient(x0, c0);
         k1 = ieee_quotient(x1, c1);
     }
 }
 __device__ __forceinline__ double mobility_recip(double c) { return recip_rn(c); }
-__device__ __forceinline__ float mobility(float x, float c, float) { return x / c; }
-__device__ __forceinline__ void mobility2(float x0, float c0, float, float x1, float c1, float, float& k0, float& k1) {
+__device__ __forceinline__ float mobility(const MC<float>&, float x, float c, float) { return x / c; }
+__device__ __forceinline__ void mobility2(float x0, float c0, float, float x1, float c1, float, bool, float& k0,
+                                          float& k1) {
     k0 = x0 / c0;
     k1 = x1 / c1;
 }
@@ -237,17 +223,22 @@ struct OpsExact {
     }
     // The far-field forms: the face fluxes and the cell update with the
     // anisotropy branches decided (kr_face and center_anisotropy both flat):
-    // a = f_a_bar, da = 0, and a dn - 0 dt is a dn (the transverse difference
+    // a = f_a_bar, da = 0, and a dn -+ 0 dt is a dn (the transverse difference
     // is finite where the test holds).  The test is conservative (far_below):
     // a pass that fails it takes the general path, whose branches decide each
     // face in the reference's rounding.
     static __device__ __forceinline__ T quarter(T d1, T c, T e) { return T(0.25) * (d1 + c - e); }
     static __device__ __forceinline__ bool far(const MC<T>& m, unsigned faces, unsigned centers) {
-        return faces < m.far_face && centers < m.far_center;
+        return (faces < m.far_face) & (centers < m.far_center);
     }
-    static __device__ __forceinline__ bool safe(const MC<T>& m, unsigned faces, unsigned centers) {
-        return max(faces, centers) < m.safe_below;
+    // the SAFE forms leave out the second ratio's own test: where a cell's
+    // phase is at least 2^-500 its differences to its neighbours are zero (as
+    // the ratio then is) or at least 2^-553, beside which a ratio below 2^-860
+    // is lost
+    static __device__ __forceinline__ bool safe(const MC<T>& m, unsigned faces, unsigned centers, T p0, T p1) {
+        return (max(faces, centers) < m.safe_below) & (min(high_word(p0) << 1, high_word(p1) << 1) >= 2 * 0x20b00000u);
     }
+    static __device__ __forceinline__ bool divides(const MC<T>& m) { return m.quotient_span == 0; }
     // of a face's differences, and of a centre's whole ones (p(i+1) - p(i-1))
     static __device__ __forceinline__ unsigned key(T dx, T dy) { return order_key(fma_t(dx, dx, dy * dy)); }
     static __device__ __forceinline__ T xface_far(const MC<T>& m, T dn) { return m.f_a_bar * (m.f_a_bar * dn); }
@@ -258,6 +249,8 @@ struct OpsExact {
     struct Cell {
         T num, c, y, lap;
     };
+    // divided outright: a reciprocal of NaN makes the quotient suspect
+    static __device__ __forceinline__ void divide(Cell& o) { o.y = T(__longlong_as_double(0x7ff8000000000000LL)); }
     static __device__ __forceinline__ void open(const MC<T>& m, T jr, T jl, T jt, T jb, T p, T uc, T ul, T ur, T up,
                                                 T um, Cell& o) {
         const T flux = (jr - jl + jt - jb) * m.inv_h2_flux;
@@ -289,12 +282,13 @@ struct OpsExact {
         return o;
     }
     static __device__ __forceinline__ void close(const MC<T>& m, const Cell& o, T& kphi, T& ku) {
-        kphi = mobility(o.num, o.c, o.y);
+        kphi = mobility(m, o.num, o.c, o.y);
         ku = fma_t(o.lap, m.d_thermal, T(0.5) * kphi);
     }
-    static __device__ __forceinline__ void close2(const MC<T>& m, const Cell& o0, const Cell& o1, T& kphi0, T& ku0,
-                                                  T& kphi1, T& ku1) {
-        mobility2(o0.num, o0.c, o0.y, o1.num, o1.c, o1.y, kphi0, kphi1);
+    // `divide`: see mobility2
+    static __device__ __forceinline__ void close2(const MC<T>& m, const Cell& o0, const Cell& o1, bool divide, T& kphi0,
+                                                  T& ku0, T& kphi1, T& ku1) {
+        mobility2(o0.num, o0.c, o0.y, o1.num, o1.c, o1.y, divide, kphi0, kphi1);
         ku0 = fma_t(o0.lap, m.d_thermal, T(0.5) * kphi0);
         ku1 = fma_t(o1.lap, m.d_thermal, T(0.5) * kphi1);
     }

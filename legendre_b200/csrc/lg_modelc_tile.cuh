@@ -638,7 +638,7 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
             const auto o1 = Ops::ocell_open(m, jr1, jl1, jt1, jbot1, C.b, C.c - C.a, D.b - B.b, c1, s1, UC, ul1,
                                             ur1, UD, UB);
             T kphi0, ku0, kphi1, ku1;
-            Ops::close2(m, o0, o1, kphi0, ku0, kphi1, ku1);
+            Ops::close2(m, o0, o1, Ops::divides(m), kphi0, ku0, kphi1, ku1);
             update(kphi0, ku0, kphi1, ku1);
             cprev = c1;
             sprev = s1;
@@ -682,13 +682,16 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
                 right_faces(fl0, fl1, fr0, fr1);
                 o0 = Ops::cell_far(m, fr0, fl0, jt0, jb, B.b, UB, ul0, ur0, UC, UA);
                 o1 = Ops::cell_far(m, fr1, fl1, jt1, jt0, C.b, UC, ul1, ur1, UD, UB);
-            } else if (!Ops::kGuarded || __all_sync(kFull, Ops::safe(m, faces, centers))) {
+            } else if (!Ops::kGuarded ||
+                       __all_sync(kFull, Ops::safe(m, faces, centers, B.b, C.b))) {
                 general(std::true_type{});
             } else {
                 general(std::false_type{});
+                Ops::divide(o0);
+                Ops::divide(o1);
             }
             T kphi0, ku0, kphi1, ku1;
-            Ops::close2(m, o0, o1, kphi0, ku0, kphi1, ku1);
+            Ops::close2(m, o0, o1, false, kphi0, ku0, kphi1, ku1);
             update(kphi0, ku0, kphi1, ku1);
         }
         store_cell(out, po, uo, off, phin0, un0, ok && own0, own0, edge_x, j, r0, n0, n1, col, lane, last_lane, sy,
