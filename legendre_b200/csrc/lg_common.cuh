@@ -93,41 +93,56 @@ __device__ __forceinline__ double log_unit_interval(double n) {
     return fma((double)e, ln2_hi, E.y) + fma((double)e, ln2_lo, p);
 }
 
-// cos x for the Box-Muller angle, x = fl(2 pi v) in (0, 2 pi], `upper` where
-// v > 1/2, to about 2e-16 relative also next to the zeros of cos: x in the
-// lower half is pi/2 + r, in the upper half 3 pi/2 + r, |r| <= pi/2, and
-// cos x = -sin r, sin r.  The centre is subtracted in two parts (the first
-// subtraction is exact next to the zero); sin r = r + r z Q(z), z = r^2, Q
-// the polynomial of degree 7 that minimises the relative error on that
-// interval (Remez exchange; 2.8e-19).
-__device__ __forceinline__ double cos_full_turn(double x, bool upper) {
-    const double c_hi = upper ? 0x1.2d97c7f3321d2p+2 : 0x1.921fb54442d18p+0;
-    const double c_lo = upper ? 0x1.a79394c9e8a0ap-53 : 0x1.1a62633145c07p-54;
-    const double r = (x - c_hi) - c_lo;
+// cos x for the Box-Muller angle, x = fl(2 pi v) in (0, 2 pi] and `top` the
+// first three bits of v, within 2.3e-16 relative, also next to the zeros of
+// cos: x = k pi/2 + r, |r| <= pi/4, with pi/2 in two parts (the first
+// subtraction is exact), then the sine r + r z S(z) or the cosine 1 + z C(z),
+// z = r^2, and the quadrant's sign.  S and C minimise the relative error on
+// that interval (Remez exchange; 3.6e-18 and 5.6e-20).  Both are evaluated: a
+// warp's lanes draw all quadrants.  One polynomial over |r| <= pi/2 takes six
+// fmas less (10080^2 4 % faster with a root within an ulp), but its rounding
+// errors are larger: the Gaussian's mean error 8.0e-17 against 7.5e-17.
+__device__ __forceinline__ double cos_full_turn(double x, int top) {
+    const int k = (top + 1) >> 1;
+    const double kd = __hiloint2double(0x43300000, k) - 0x1p52;
+    const double r = fma(-kd, 0x1.1a62633145c07p-54, fma(-kd, 0x1.921fb54442d18p+0, x));
     const double z = r * r;
-    double q = 0x1.8829a29fbb6b6p-49;
-    q = fma(q, z, -0x1.ae431d97313e9p-41);
-    q = fma(q, z, 0x1.6123cb2907df4p-33);
-    q = fma(q, z, -0x1.ae6454cb57936p-26);
-    q = fma(q, z, 0x1.71de3a5287c8ap-19);
-    q = fma(q, z, -0x1.a01a01a0148bdp-13);
-    q = fma(q, z, 0x1.11111111110c1p-7);
-    q = fma(q, z, -0x1.5555555555555p-3);
-    const double s = fma(r * z, q, r);
-    return __hiloint2double(__double2hiint(s) ^ (upper ? 0 : 0x80000000), __double2loint(s));
+    double s = 0x1.5d8fba92fea51p-33;
+    s = fma(s, z, -0x1.ae5e5a4426ab5p-26);
+    s = fma(s, z, 0x1.71de3567738e7p-19);
+    s = fma(s, z, -0x1.a01a019bfd844p-13);
+    s = fma(s, z, 0x1.111111110f7cdp-7);
+    s = fma(s, z, -0x1.5555555555548p-3);
+    s = fma(r * z, s, r);
+    double c = -0x1.8fa4800fb4bcbp-37;
+    c = fma(c, z, 0x1.1ee9d783e31abp-29);
+    c = fma(c, z, -0x1.27e4f7ea7e667p-22);
+    c = fma(c, z, 0x1.a01a019c83f08p-16);
+    c = fma(c, z, -0x1.6c16c16c14f8ep-10);
+    c = fma(c, z, 0x1.555555555554bp-5);
+    c = fma(c, z, -0.5);
+    c = fma(z, c, 1.0);
+    const double v = (k & 1) ? s : c;
+    return __hiloint2double(__double2hiint(v) ^ (((k + 1) & 2) << 30), __double2loint(v));
 }
 
-// sqrt w for w = 0 or 2^-60 < w < 2^60, within an ulp: g = w y with y the
-// hardware's approximation of 1 / sqrt(w) (better than 2^-19), then the cubic
-// Householder step g (1 + e/2 + 3 e^2 / 8), e = 1 - g y.  A zero of either
-// sign gives itself (the approximation's infinity is made finite).
+// sqrt w for w = 0 or 2^-60 < w < 2^60, correctly rounded: g = w y and h = y /
+// 2 with y the hardware's approximation of 1 / sqrt(w) (better than 2^-19),
+// the cubic Householder step (1 + e/2 + 3 e^2 / 8), e = 1 - g y, on both, and
+// one correction with the exact residual, g + (w - g^2) h (Markstein, IBM J.
+// Res. Dev. 34, 1990).  A zero of either sign gives itself (the
+// approximation's infinity is made finite).
 __device__ __forceinline__ double sqrt_radius(double w) {
     double y;
     asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(w));
-    y = __hiloint2double(min(__double2hiint(y) & 0x7fffffff, 0x7fe00000), 0);
-    const double g = w * y;
+    const int hy = min(__double2hiint(y) & 0x7fffffff, 0x7fe00000);
+    y = __hiloint2double(hy, 0);
+    double g = w * y, h = __hiloint2double(hy - 0x00100000, 0);
     const double e = fma(-g, y, 1.0);
-    return fma(g * e, fma(e, 0.375, 0.5), g);
+    const double s = e * fma(e, 0.375, 0.5);
+    g = fma(g, s, g);
+    h = fma(h, s, h);
+    return fma(fma(-g, g, w), h, g);
 }
 
 // Box-Muller cosine branch from one key (src/util/rng.rs:43-49): the
@@ -140,7 +155,7 @@ __device__ __forceinline__ double standard_normal(uint64_t key) {
     const double nu = (double)((a >> 11) + 1), nv = (double)((b >> 11) + 1);
     // fl(2 pi v): the power of two scales exactly
     const double x = nv * (kTau * (1.0 / 9007199254740992.0));
-    return sqrt_radius(-2.0 * log_unit_interval(nu)) * cos_full_turn(x, (int64_t)b < 0);
+    return sqrt_radius(-2.0 * log_unit_interval(nu)) * cos_full_turn(x, (int)(b >> 61));
 }
 
 // Single-precision Gaussian from the same two uniforms, for the FP32 path.
