@@ -562,12 +562,16 @@ __device__ __forceinline__ void strip_unit_pair(const typename Ops::Params& m, u
         T c0 = T(0), s0 = T(0), c1 = T(0), s1 = T(0);  // multi-grain: frames of rows j and j+1
         if constexpr (ORIENT) {
             const int64_t ci = (int64_t)j * n0 + ccol;
-            const int64_t p2 = ci + (int64_t)(min(j + 2, n1 - 1) - j) * n0;  // the next pass's frames
-            const int64_t p3 = ci + (int64_t)(min(j + 3, n1 - 1) - j) * n0;
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p2));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p2));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p3));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p3));
+            if constexpr (sizeof(T) == 8) {
+                // the next pass's frames (2520^2 167 -> 165 us a step; FP32,
+                // whose passes are shorter on instructions, 92 -> 97)
+                const int64_t p2 = ci + (int64_t)(min(j + 2, n1 - 1) - j) * n0;
+                const int64_t p3 = ci + (int64_t)(min(j + 3, n1 - 1) - j) * n0;
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p2));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p2));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + p3));
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(trig_b + ncells + p3));
+            }
             c0 = __ldg(trig_b + ci);
             s0 = __ldg(trig_b + ncells + ci);
             c1 = __ldg(trig_b + ci + n0);
@@ -832,24 +836,36 @@ constexpr int strip_group() {
     return PAIR ? 2 : (sizeof(T) == 4 && ORIENT ? 4 : 1);
 }
 
-// Rows per work unit, where the caller leaves them open: the power of two up
-// to 32 (one batch of boundary faces per unit) that minimises the step's
-// length.  A warp spends about two rows' time on starting a unit, and a row's
-// time hardly depends on how many warps share the SM until the resident warps
-// (`slots`) are all busy; from there on the units queue (FP32 rows are short
-// enough to feel the queue from about three quarters on).  FP64 paired rows
-// at 2, 4, 8, 16 rows a unit: 64^2 4.8, 6.8, 11.0, 19.4 us a step; 512^2 8.6,
-// 8.4, 11.2, 19.5; 1008^2 25.0, 21.2, 19.8, 25.1; 2048^2 98, 77, 67, 63.
-template <class T>
+// Rows per work unit, where the caller leaves them open: of a few heights up
+// to 32 (one batch of boundary faces per unit) the one that minimises the
+// step's length.  A warp spends about two rows' time on starting a unit, and a
+// row's time hardly depends on how many warps share the SM until the resident
+// warps (`slots`) are all busy; from there on the units queue.
+//
+// FP64, and FP32 axis-aligned in one state: powers of two; FP32 rows are short enough to feel the
+// queue from about three quarters on.  FP64 paired rows at 2, 4, 8, 16 rows a
+// unit: 64^2 4.8, 6.8, 11.0, 19.4 us a step; 512^2 8.6, 8.4, 11.2, 19.5; 1008^2
+// 25.0, 21.2, 19.8, 25.1; 2048^2 98, 77, 67, 63.
+//
+// FP32 multi-grain and batched (TAILED): a single wave runs as fast as its units, but from
+// one wave on half a unit's time is spent on the last, partly filled one, so
+// heights between the powers of two pay.  With noise at 6, 8, 12, 16, 32 rows:
+// 500^2 in blocks of 100^2 9.4, 11.3, 10.5, 12.5, 21.6 us a step; 1500^2 50.3,
+// 47.5, 46.8, 53.2, 63.1; 2520^2 (126^2) 95.7, 91.0, 89.5, 84.8, 92.3.  Within
+// 1 % of the best height on average over 500^2 to 3072^2, 7 % at most; the
+// rule above chose up to 30 % off.  48 instances of 144^2 in blocks of 48^2
+// 25.0 -> 24.1 us a step.
+template <class T, bool TAILED>
 inline int strip_auto_rows(const CartTopo& topo, int strips, int64_t slots) {
     const int n1 = topo.n[1];
-    const double queue = sizeof(T) == 8 ? 1.0 : 1.36;
     int best = 2;
     double best_cost = 0.0;
-    for (int rows = 32; rows >= 2; rows /= 2) {
+    for (int rows : {32, 24, 20, 16, 12, 10, 8, 6, 4, 2}) {
+        if (!TAILED && (rows & (rows - 1)) != 0) continue;
         const int h = std::min(rows, n1);
-        const double units = (double)topo.nblocks * strips * ((n1 + h - 1) / h);
-        const double cost = (h + 2) * std::max(1.0, queue * units / (double)slots);
+        const double waves = (double)topo.nblocks * strips * ((n1 + h - 1) / h) / (double)slots;
+        const double cost = TAILED ? (h + 1.5) * (waves <= 1.0 ? 1.0 : waves + 0.5)
+                                   : (h + 2) * std::max(1.0, (sizeof(T) == 8 ? 1.0 : 1.36) * waves);
         if (best_cost == 0.0 || cost < best_cost) {
             best_cost = cost;
             best = h;
@@ -861,12 +877,12 @@ inline int strip_auto_rows(const CartTopo& topo, int strips, int64_t slots) {
 // work decomposition of a launch: units of (block, strip, row chunk) of
 // g.rows rows (at most 32; 0: chosen as above), a whole number of groups of
 // nb rows; true when the block is lower than the row group (the TAIL kernels)
-template <class T>
+template <class T, bool TAILED = false>
 inline bool strip_plan(TileArgs& g, int nb, int ctas_per_sm) {
     const int n0 = g.topo.n[0], n1 = g.topo.n[1];
     g.strips = (n0 + 31) / 32;
     const int64_t slots = (int64_t)device_sm_count() * ctas_per_sm * 8;
-    int rows = g.rows > 0 ? g.rows : strip_auto_rows<T>(g.topo, g.strips, slots);
+    int rows = g.rows > 0 ? g.rows : strip_auto_rows<T, TAILED>(g.topo, g.strips, slots);
     rows = std::max(1, std::min(std::min(rows, 32), n1));
     if (n1 >= nb) rows = std::max(nb, rows / nb * nb);
     g.rows = rows;
@@ -906,7 +922,7 @@ inline dim3 strip_ctas(const TileArgs& g, int ctas_per_sm) {
 // PAIR: the paired rows (256 instances of 256^2, FP32: 102.5 against 79.8 Gcell/s)
 template <class T, class Ops, bool NOISE, int MINB, bool PAIR = false>
 cudaError_t launch_strip_batch(const T* in, T* out, TileArgs g, BatchArgs bt, T dt, T scale_amp, cudaStream_t s) {
-    const bool tail = strip_plan<T>(g, strip_group<T, false, PAIR>(), MINB);
+    const bool tail = strip_plan<T, sizeof(T) == 4>(g, strip_group<T, false, PAIR>(), MINB);
     const dim3 grid = strip_ctas(g, MINB);
     const typename Ops::Params m{};
     if (tail) {
@@ -947,7 +963,7 @@ cudaError_t launch_strip_minb(const T* in, T* out, TileArgs g, const typename Op
 template <class T, class Ops, bool NOISE, int MINB, bool PAIR = false>
 cudaError_t launch_strip_oriented(const T* in, T* out, TileArgs g, const typename Ops::Params& m, T dt, T scale_amp,
                                   OrientArgs oa, cudaStream_t s) {
-    const bool tail = strip_plan<T>(g, strip_group<T, true, PAIR>(), MINB);
+    const bool tail = strip_plan<T, sizeof(T) == 4>(g, strip_group<T, true, PAIR>(), MINB);
     const dim3 grid = strip_ctas(g, MINB);
     if (tail) {  // blocks lower than the row group: single rows
         return strip_launch(modelc_strip_kernel<T, Ops, NOISE, MINB, 0, 1, false, true, true>, grid, s, in, out, g, m, dt, scale_amp, BatchArgs{}, oa, RkArgs<T>{});
