@@ -547,11 +547,12 @@ int lg_heat_fe_run(lg_state* st, int field, double kappa, double dt, int64_t nst
     // interiors, ghosts filled once at the end; 1-D: the push kernel, one step
     // per launch, which keeps the ghosts valid
     const bool march = lg::heat_march_supported(topo, L);
+    lg::HeatPlan plans[2];
     auto launch = [&](int steps) -> int {
         const double* in = static_cast<const double*>(st->arena[st->cur]);
         double* out = static_cast<double*>(st->arena[st->cur ^ 1]);
         cudaError_t e = march ? lg::launch_heat_march_fe(steps, in, out, topo, L, field, st->grid->periodic, kappa,
-                                                         dt, inv_h2, ctx->stream)
+                                                         dt, inv_h2, plans[steps - 1], ctx->stream)
                               : lg::launch_heat_step(in, out, topo, L, field, kappa, dt, inv_h2, ctx->stream);
         ctx->launches++;
         if (e != cudaSuccess) return cuda_fail(ctx, e, "heat step launch");
@@ -876,16 +877,17 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
     double* k3 = static_cast<double*>(st->rk[2]);
     double* t0 = static_cast<double*>(st->rk[3]);
     double* t1 = static_cast<double*>(st->rk[4]);
+    lg::HeatPlan plans[2];
     auto step = [&]() -> int {
         const double* y = static_cast<const double*>(st->arena[st->cur]);
         double* out = static_cast<double*>(st->arena[st->cur ^ 1]);
         cudaError_t e;
         if (march) {  // 2-D and 3-D: two stages per launch, k1 and k2 hold y + c k2 and the running sum
             e = lg::launch_heat_march_rk4(0, y, k1, nullptr, k2, topo, L, field, st->grid->periodic, kappa, dt,
-                                          inv_h2, ctx->stream);
+                                          inv_h2, plans[0], ctx->stream);
             if (e == cudaSuccess)
                 e = lg::launch_heat_march_rk4(1, k1, out, y, k2, topo, L, field, st->grid->periodic, kappa, dt,
-                                              inv_h2, ctx->stream);
+                                              inv_h2, plans[1], ctx->stream);
             ctx->launches += 2;
             if (e != cudaSuccess) return cuda_fail(ctx, e, "heat RK4 launch");
             st->cur ^= 1;

@@ -4,8 +4,10 @@
 // reference's operand order (finite_difference.rs:49-67, euler.rs:51-53,
 // rk4.rs:40-79), so the results are the reference's bits.
 #include <algorithm>
+#include <atomic>
 
 #include "lg_common.cuh"
+#include "lg_heat_plan.h"
 #include "lg_kernels.h"
 
 namespace lg {
@@ -17,8 +19,6 @@ namespace {
 // s3 k2).  kRkB: stages 3 and 4 (in = y + c k2 of kRkA, y, aux; out = ((aux +
 // s3 k3) + s6 k4).  The running sum aux is rk4.rs's chain of axpys in its
 // order, so no k is ever stored.
-constexpr int kMaxPlanes = 256;  // planes a CTA marches over, at most
-
 enum HeatForm { kFe1, kFe2, kRkA, kRkB };
 
 struct HeatArgs {
@@ -289,36 +289,35 @@ __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, M
     }
 }
 
-// Planes per CTA: the number of chunks whose waves of resident CTAs spend
-// the fewest plane iterations, a CTA running zc + 2 H planes plus about four
-// iterations of start-up (address set-up and the first loads' latency).
-int march_planes(int64_t tiles, int planes, int halo, int64_t slots) {
-    int64_t best = -1;
-    int best_zc = std::min(planes, kMaxPlanes);
-    for (int chunks = (planes + kMaxPlanes - 1) / kMaxPlanes; chunks <= planes; ++chunks) {
-        const int zc = (planes + chunks - 1) / chunks;
-        const int64_t ctas = tiles * ((planes + zc - 1) / zc);
-        const int64_t cost = (ctas + slots - 1) / slots * (zc + 2 * halo + 4);
-        if (best < 0 || cost < best) {
-            best = cost;
-            best_zc = zc;
-        }
-        if (best >= 0 && tiles * chunks > 64 * slots) break;  // many waves: the halo planes only add from here on
-    }
-    return best_zc;
+// CTAs of a form that an SM holds, asked for once
+template <int FORM, int WX, int TR, int R, int PITCH, int MINB, class Off>
+cudaError_t march_occupancy(int& per_sm) {
+    static std::atomic<int> known{0};
+    per_sm = known.load(std::memory_order_relaxed);
+    if (per_sm > 0) return cudaSuccess;
+    auto* kernel = heat_march_kernel<FORM, WX, TR, R, PITCH, MINB, Off>;
+    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+        &per_sm, kernel, MarchTile<FORM, WX, TR, R, PITCH>::kThreads, 0);
+    if (e != cudaSuccess) return e;
+    per_sm = std::max(per_sm, 1);
+    known.store(per_sm, std::memory_order_relaxed);
+    return cudaSuccess;
 }
 
 template <int FORM, int WX, int TR, int R, int PITCH, int MINB, class Off>
-cudaError_t launch_march(HeatArgs a, cudaStream_t s) {
+cudaError_t launch_march(HeatArgs a, HeatPlan& plan, cudaStream_t s) {
     using G = MarchTile<FORM, WX, TR, R, PITCH>;
     auto* kernel = heat_march_kernel<FORM, WX, TR, R, PITCH, MINB, Off>;
-    int per_sm = 0;
-    const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, G::kThreads, 0);
-    if (e != cudaSuccess) return e;
     a.tiles_x = (a.N[0] + G::kOX - 1) / G::kOX;
     a.tiles_y = (a.N[1] + G::kOY - 1) / G::kOY;
     const int64_t tiles = (int64_t)a.tiles_x * a.tiles_y;
-    a.zc = march_planes(tiles, a.N[2], G::kH, (int64_t)device_sm_count() * std::max(per_sm, 1));
+    if (plan.planes == 0) {
+        int per_sm = 0;
+        const cudaError_t e = march_occupancy<FORM, WX, TR, R, PITCH, MINB, Off>(per_sm);
+        if (e != cudaSuccess) return e;
+        plan.planes = march_planes(tiles, a.N[2], G::kH, (int64_t)device_sm_count() * per_sm);
+    }
+    a.zc = plan.planes;
     const int64_t ctas = tiles * ((a.N[2] + a.zc - 1) / a.zc);
     if (ctas > (int64_t)0x7fffffff) return cudaErrorInvalidConfiguration;
     cudaLaunchConfig_t cfg = {};
@@ -334,20 +333,21 @@ cudaError_t launch_march(HeatArgs a, cudaStream_t s) {
 }
 
 template <int FORM, class Off>
-cudaError_t launch_form(int D, const HeatArgs& a, cudaStream_t s) {
-    if (D == 2) return launch_march<FORM, 128, 1, 1, 128, 4, Off>(a, s);
+cudaError_t launch_form(int D, const HeatArgs& a, HeatPlan& plan, cudaStream_t s) {
+    if (D == 2) return launch_march<FORM, 128, 1, 1, 128, 4, Off>(a, plan, s);
     // 28 x 28 columns and four rows a thread, or, where such tiles leave SMs
     // idle, 32 x 16 columns and two rows a thread, whose iterations are
     // shorter (96^3: 4.7 against 6.1 us a step; 512^3: 445 against 396)
     const int64_t cells = (int64_t)a.N[0] * a.N[1] * a.N[2];
-    if (cells >= 4000000) return launch_march<FORM, 32, 8, 4, 32, 2, Off>(a, s);
-    return launch_march<FORM, 36, 10, 2, 42, 2, Off>(a, s);
+    if (cells >= 4000000) return launch_march<FORM, 32, 8, 4, 32, 2, Off>(a, plan, s);
+    return launch_march<FORM, 36, 10, 2, 42, 2, Off>(a, plan, s);
 }
 
 template <int FORM>
-cudaError_t launch_form(int D, const HeatArgs& a, cudaStream_t s) {
+cudaError_t launch_form(int D, const HeatArgs& a, HeatPlan& plan, cudaStream_t s) {
     // a column's byte offset inside one layer of blocks: 32 bits where they hold it
-    return a.bstr[2] < (int64_t)1 << 28 ? launch_form<FORM, uint32_t>(D, a, s) : launch_form<FORM, int64_t>(D, a, s);
+    return a.bstr[2] < (int64_t)1 << 28 ? launch_form<FORM, uint32_t>(D, a, plan, s)
+                                       : launch_form<FORM, int64_t>(D, a, plan, s);
 }
 
 HeatArgs march_args(const CartTopo& topo, const SlabLayout& L, int field, const int periodic[3], double kappa,
@@ -388,17 +388,17 @@ bool heat_march_supported(const CartTopo& topo, const SlabLayout& L) {
 
 cudaError_t launch_heat_march_fe(int steps, const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                  int field, const int periodic[3], double kappa, double dt, const double inv_h2[3],
-                                 cudaStream_t s) {
+                                 HeatPlan& plan, cudaStream_t s) {
     HeatArgs a = march_args(topo, L, field, periodic, kappa, inv_h2);
     a.in = in + (int64_t)field * L.slab_stride;
     a.out = out + (int64_t)field * L.slab_stride;
     a.c1 = a.c2 = dt;
-    return steps == 2 ? launch_form<kFe2>(topo.D, a, s) : launch_form<kFe1>(topo.D, a, s);
+    return steps == 2 ? launch_form<kFe2>(topo.D, a, plan, s) : launch_form<kFe1>(topo.D, a, plan, s);
 }
 
 cudaError_t launch_heat_march_rk4(int half, const double* in, double* out, const double* y, double* aux,
                                   const CartTopo& topo, const SlabLayout& L, int field, const int periodic[3],
-                                  double kappa, double dt, const double inv_h2[3], cudaStream_t s) {
+                                  double kappa, double dt, const double inv_h2[3], HeatPlan& plan, cudaStream_t s) {
     HeatArgs a = march_args(topo, L, field, periodic, kappa, inv_h2);
     const int64_t f = (int64_t)field * L.slab_stride;
     a.in = in + f;
@@ -408,12 +408,12 @@ cudaError_t launch_heat_march_rk4(int half, const double* in, double* out, const
     if (half == 0) {
         a.aux = aux + f;
         a.c1 = a.c2 = 0.5 * dt;  // rk4.rs:57
-        return launch_form<kRkA>(topo.D, a, s);
+        return launch_form<kRkA>(topo.D, a, plan, s);
     }
     a.y = y + f;
     a.aux_in = aux + f;
     a.c1 = dt;
-    return launch_form<kRkB>(topo.D, a, s);
+    return launch_form<kRkB>(topo.D, a, plan, s);
 }
 
 }  // namespace lg

@@ -1,0 +1,35 @@
+// How the marching heat kernel (lg_heat.cu) divides a grid.  Host code only.
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+namespace lg {
+
+constexpr int kMaxPlanes = 256;  // planes a CTA marches over, at most
+
+// Planes per CTA: of the heights that some number of chunks gives, the one
+// whose waves of resident CTAs (`slots`) spend the fewest plane iterations, a
+// CTA running zc + 2 halo planes plus about four iterations of start-up
+// (address set-up and the first loads' latency).  It looks at no more than 2
+// sqrt(planes) heights, 256 in all, and once a run: one chunk count after the
+// other at every launch took 5 us on 1425 x 1001, where a launch takes 10.7,
+// and 165 on 128 x 100000.
+inline int march_planes(int64_t tiles, int planes, int halo, int64_t slots) {
+    int64_t best = -1;
+    int best_zc = std::min(planes, kMaxPlanes);
+    for (int zc = best_zc; zc >= 1; --zc) {
+        const unsigned chunks = ((unsigned)planes + zc - 1) / zc;
+        zc = (int)(((unsigned)planes + chunks - 1) / chunks);  // the lowest height with as many chunks
+        const int64_t ctas = tiles * chunks;
+        const int64_t cost = (ctas + slots - 1) / slots * (zc + 2 * halo + 4);
+        if (best < 0 || cost < best) {
+            best = cost;
+            best_zc = zc;
+        }
+        if (ctas > 64 * slots) break;  // many waves: the halo planes only add from here on
+    }
+    return best_zc;
+}
+
+}  // namespace lg

@@ -43,14 +43,19 @@ cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo
 // `out` gets interiors only (its ghost columns are scratch).  RungeKutta4:
 // half 0 reads the state from `in` and leaves y + dt/2 k2 in `out` and the
 // running sum of the axpys in `aux`; half 1 reads those from `in` and `aux`
-// and the state from `y`.  Bit-identical to the reference's steps.
+// and the state from `y`.  Bit-identical to the reference's steps.  `plan` is
+// the division of the grid, made by the first launch of a run (one for each
+// form) and kept by the caller for the others.
+struct HeatPlan {
+    int planes = 0;  // planes per CTA; 0: not made yet
+};
 bool heat_march_supported(const CartTopo& topo, const SlabLayout& L);
 cudaError_t launch_heat_march_fe(int steps, const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                  int field, const int periodic[3], double kappa, double dt, const double inv_h2[3],
-                                 cudaStream_t s);
+                                 HeatPlan& plan, cudaStream_t s);
 cudaError_t launch_heat_march_rk4(int half, const double* in, double* out, const double* y, double* aux,
                                   const CartTopo& topo, const SlabLayout& L, int field, const int periodic[3],
-                                  double kappa, double dt, const double inv_h2[3], cudaStream_t s);
+                                  double kappa, double dt, const double inv_h2[3], HeatPlan& plan, cudaStream_t s);
 
 // (a) fused Model C Euler-Maruyama step, FP64, bit-exact to the reference.
 // Reads phi (field 0) and u (field 1) from `in`, writes both to `out` with
