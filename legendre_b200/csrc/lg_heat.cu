@@ -304,43 +304,81 @@ cudaError_t march_occupancy(int& per_sm) {
     return cudaSuccess;
 }
 
-template <int FORM, int WX, int TR, int R, int PITCH, int MINB, class Off>
-cudaError_t launch_march(HeatArgs a, HeatPlan& plan, cudaStream_t s) {
+// one tile shape: what it would cost (`factor`: what march_cost misses of it),
+// and the launch
+template <int FORM, class Off, int WX, int TR, int R, int PITCH, int MINB>
+struct March {
     using G = MarchTile<FORM, WX, TR, R, PITCH>;
-    auto* kernel = heat_march_kernel<FORM, WX, TR, R, PITCH, MINB, Off>;
-    a.tiles_x = (a.N[0] + G::kOX - 1) / G::kOX;
-    a.tiles_y = (a.N[1] + G::kOY - 1) / G::kOY;
-    const int64_t tiles = (int64_t)a.tiles_x * a.tiles_y;
-    if (plan.planes == 0) {
+    static void tiles(HeatArgs& a) {
+        a.tiles_x = (a.N[0] + G::kOX - 1) / G::kOX;
+        a.tiles_y = (a.N[1] + G::kOY - 1) / G::kOY;
+    }
+    static cudaError_t consider(int tile, double factor, HeatArgs a, HeatPlan& plan) {
         int per_sm = 0;
         const cudaError_t e = march_occupancy<FORM, WX, TR, R, PITCH, MINB, Off>(per_sm);
         if (e != cudaSuccess) return e;
-        plan.planes = march_planes(tiles, a.N[2], G::kH, (int64_t)device_sm_count() * per_sm);
+        tiles(a);
+        const int64_t n = (int64_t)a.tiles_x * a.tiles_y, sms = device_sm_count();
+        const int zc = march_planes(n, a.N[2], G::kH, sms * per_sm);
+        const double cost = factor * march_cost(n, a.N[2], zc, G::kH, sms, per_sm, G::kThreads, R);
+        if (plan.tile < 0 || cost < plan.cost) plan = HeatPlan{tile, zc, cost};
+        return cudaSuccess;
     }
-    a.zc = plan.planes;
-    const int64_t ctas = tiles * ((a.N[2] + a.zc - 1) / a.zc);
-    if (ctas > (int64_t)0x7fffffff) return cudaErrorInvalidConfiguration;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(G::kThreads);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, a);
-}
+    static cudaError_t launch(HeatArgs a, const HeatPlan& plan, cudaStream_t s) {
+        tiles(a);
+        a.zc = plan.planes;
+        const int64_t ctas = (int64_t)a.tiles_x * a.tiles_y * ((a.N[2] + a.zc - 1) / a.zc);
+        if (ctas > (int64_t)0x7fffffff) return cudaErrorInvalidConfiguration;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3(G::kThreads);
+        cfg.stream = s;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, heat_march_kernel<FORM, WX, TR, R, PITCH, MINB, Off>, a);
+    }
+};
 
+// The tile shapes (window columns, thread rows, rows a thread) and the rule
+// between them, march_cost.  2-D: a row of 128.  3-D: 32 x 16 columns with two
+// rows a thread; Euler steps also 28 x 28 with four, where tiles are many
+// (RungeKutta4 keeps two more arrays a row in registers: 256^3 375 us a step
+// against 313); 8 x 80, 8 x 8 and (Euler) 60 x 8 for grids narrow in x, in both
+// or in y, of which the others would fill a part of a window: 8 x 512 x 512 23.9
+// -> 9.9 us a step, 8 x 8 x 4096 7.3 -> 4.3, 512 x 8 x 512 13.5 -> 9.4.
 template <int FORM, class Off>
 cudaError_t launch_form(int D, const HeatArgs& a, HeatPlan& plan, cudaStream_t s) {
-    if (D == 2) return launch_march<FORM, 128, 1, 1, 128, 4, Off>(a, plan, s);
-    // 28 x 28 columns and four rows a thread, or, where such tiles leave SMs
-    // idle, 32 x 16 columns and two rows a thread, whose iterations are
-    // shorter (96^3: 4.7 against 6.1 us a step; 512^3: 445 against 396)
-    const int64_t cells = (int64_t)a.N[0] * a.N[1] * a.N[2];
-    if (cells >= 4000000) return launch_march<FORM, 32, 8, 4, 32, 2, Off>(a, plan, s);
-    return launch_march<FORM, 36, 10, 2, 42, 2, Off>(a, plan, s);
+    constexpr bool kEuler = FORM == kFe1 || FORM == kFe2, kNarrow = sizeof(Off) == 4;
+    using Row = March<FORM, Off, 128, 1, 1, 128, 4>;
+    using Few = March<FORM, Off, 36, 10, 2, 42, 2>;
+    using Wide = March<FORM, Off, 32, 8, 4, 32, 2>;
+    using NarrowX = March<FORM, Off, 12, 21, 4, 15, 2>;
+    using Narrow = March<FORM, Off, 12, 3, 4, 15, 8>;
+    using NarrowY = March<FORM, Off, 64, 3, 4, 64, 3>;
+    if (plan.tile < 0) {
+        cudaError_t e = D == 2 ? Row::consider(0, 1.0, a, plan) : Few::consider(1, 1.0, a, plan);
+        if constexpr (kEuler)
+            if (e == cudaSuccess && D == 3) e = Wide::consider(2, 1.0, a, plan);
+        if constexpr (kNarrow) {
+            if (e == cudaSuccess && D == 3) e = NarrowX::consider(3, kEuler ? 1.0 : 1.25, a, plan);
+            if (e == cudaSuccess && D == 3) e = Narrow::consider(4, 1.0, a, plan);
+            if constexpr (kEuler)
+                if (e == cudaSuccess && D == 3) e = NarrowY::consider(5, 1.15, a, plan);
+        }
+        if (e != cudaSuccess) return e;
+    }
+    if constexpr (kEuler)
+        if (plan.tile == 2) return Wide::launch(a, plan, s);
+    if constexpr (kNarrow) {
+        if (plan.tile == 3) return NarrowX::launch(a, plan, s);
+        if (plan.tile == 4) return Narrow::launch(a, plan, s);
+        if constexpr (kEuler)
+            if (plan.tile == 5) return NarrowY::launch(a, plan, s);
+    }
+    return plan.tile == 0 ? Row::launch(a, plan, s) : Few::launch(a, plan, s);
 }
 
 template <int FORM>

@@ -47,7 +47,9 @@ cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo
 // the division of the grid, made by the first launch of a run (one for each
 // form) and kept by the caller for the others.
 struct HeatPlan {
-    int planes = 0;  // planes per CTA; 0: not made yet
+    int tile = -1;  // the tile shape; negative: not made yet
+    int planes = 0;  // planes per CTA
+    double cost = 0.0;
 };
 bool heat_march_supported(const CartTopo& topo, const SlabLayout& L);
 cudaError_t launch_heat_march_fe(int steps, const double* in, double* out, const CartTopo& topo, const SlabLayout& L,

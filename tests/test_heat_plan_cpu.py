@@ -1,5 +1,6 @@
 """The plan of the marching heat kernel (lg_heat_plan.h) on the CPU: the planes
-per CTA cost no more than the best of every chunk count, found in few tries."""
+per CTA cost no more than the best of every chunk count, found in few tries,
+and a tile that the grid fills costs less than one it does not."""
 import shutil
 import subprocess
 from pathlib import Path
@@ -36,6 +37,11 @@ int main() {
     int sum = 0;
     for (int i = 0; i < 10; ++i) sum += march_planes(1, 1 << 30, 2, 1 << 26);
     const double s = std::chrono::duration<double>(std::chrono::steady_clock::now() - t).count();
+    // 8 cells of 8 or of 32 columns, the same threads and rows
+    const int64_t narrow = 64, wide = 16;
+    if (!(march_cost(narrow / 8, 512, march_planes(narrow / 8, 512, 2, 296), 2, 148, 2, 252, 4) <
+          march_cost(wide * 2, 512, march_planes(wide * 2, 512, 2, 296), 2, 148, 2, 384, 2)))
+        ++wrong;
     std::printf("%d wrong, %g s (%d)\n", wrong, s, sum);
     return wrong != 0 || s > 5e-3;
 }
