@@ -206,7 +206,8 @@ class AmrSimulation:
         return self.fields.index(f) if isinstance(f, str) else int(f)
 
     def get(self, f) -> List[np.ndarray]:
-        """Per-block ghost-inclusive slabs of field f, each (ny+2, nx+2)."""
+        """Per-block ghost-inclusive slabs of field f, each (ny+2, nx+2): arrays of one new buffer
+        (a copy each costs more than the read: 2048^2 in 64 blocks 16 ms, 7.8 without)."""
         n = C.c_int64()
         N.check(N.lib.lg_amr_sim_field_len(self.handle, C.byref(n)))
         flat = np.empty(n.value)
@@ -216,7 +217,7 @@ class AmrSimulation:
         for lv, lo, hi in self.patches():
             nx, ny = hi[0] - lo[0], hi[1] - lo[1]
             k = (nx + 2) * (ny + 2)
-            out.append(flat[off:off + k].reshape(ny + 2, nx + 2).copy())
+            out.append(flat[off:off + k].reshape(ny + 2, nx + 2))
             off += k
         return out
 

@@ -92,11 +92,12 @@ __global__ void amr_restrict_kernel(double* C, const double* F, const RestrictOp
 
 // One field's slabs, each level's from its current buffer, packed one after
 // the other in block order: what a read-back hands out, so that it crosses to
-// the host in one copy of that field alone.  Bound: the copy to the host (the
-// kernel moves 16 B an entry in HBM, a few us; a 512^2 base with three levels
-// holds 3 MB a field).  A field read through the Python class, its 611 blocks
-// handed out as arrays: 2.2 ms with every field's slabs copied to the host and
-// picked there, 1.7 with this.
+// the host in one copy of that field alone.  A block is spread over
+// gridDim.y CTAs, one for every 4096 entries of the largest block.  Bound: the
+// copy to the host (the kernel moves 16 B an entry in HBM; a 512^2 base with
+// three levels holds 3 MB a field).  Read-back of one field: a block of 1024^2
+// 1.7 ms with every field's slabs copied to the host and picked there, 1.25
+// packed by one CTA, 0.50 as here; 64 blocks of 64^2 0.50, 0.18, 0.18.
 constexpr int kPackLevels = 32;  // deeper hierarchies are picked on the host
 struct PackArgs {
     const double* level[kPackLevels];
@@ -110,7 +111,8 @@ __global__ void __launch_bounds__(256) amr_pack_kernel(const BlockDesc* __restri
         const double* v = a.level[b.level] + b.off + field * b.stride;
         double* o = out + to[k];
         const int64_t n = (int64_t)(b.nx + 2) * (b.ny + 2);
-        for (int64_t i = threadIdx.x; i < n; i += blockDim.x) o[i] = v[i];
+        for (int64_t i = (int64_t)blockIdx.y * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.y * blockDim.x)
+            o[i] = v[i];
     }
 }
 
@@ -1702,8 +1704,10 @@ int lg_amr_sim_get_field(lg_amr_sim* s, int field, double* host, int64_t nelem) 
         PackArgs a{};
         for (int l = 0; l < levels; ++l) a.level[l] = s->arena[s->cur[l]];
         const int nblocks = (int)s->plans.blocks.size();
-        amr_pack_kernel<<<(unsigned)std::min(nblocks, 65535), 256, 0, st>>>(s->tab.blocks, s->tab.pack, nblocks, a,
-                                                                           field, s->d_pack);
+        int64_t largest = 0;
+        for (const auto& b : s->plans.blocks) largest = std::max(largest, (int64_t)(b.nx + 2) * (b.ny + 2));
+        const dim3 grid((unsigned)std::min(nblocks, 65535), (unsigned)std::min<int64_t>((largest + 4095) / 4096, 65535));
+        amr_pack_kernel<<<grid, 256, 0, st>>>(s->tab.blocks, s->tab.pack, nblocks, a, field, s->d_pack);
         lg::abi_count_launch(s->ctx, 1);
         AMR_CUDA(s, cudaGetLastError());
         AMR_CUDA(s, cudaMemcpyAsync(host, s->d_pack, (size_t)n * sizeof(double), cudaMemcpyDeviceToHost, st));
