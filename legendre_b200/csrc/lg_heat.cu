@@ -161,13 +161,13 @@ __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, M
     auto put = [](double* p, int64_t plane, Off o) {
         return reinterpret_cast<double*>(reinterpret_cast<char*>(p) + plane + o);
     };
-    // programmatic dependent launch: wait for the predecessor's writes, then
-    // let the next launch become resident (not before the wait: it must not
-    // start while the launch before this one still fills an L1 it will read)
+    // programmatic dependent launch: wait until the predecessor is complete
+    // and its writes visible, then let the next launch become resident (not
+    // before the wait: its CTAs would hold slots while two launches still run)
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-    // loads bypass L1 (an element is read once per CTA)
+    // loads bypass L1: an element is read once per CTA
     double U[UR][R], V[3][R], S[2][R], Y[2][R], X[2][R];
     const int64_t* po = plane_off;
 #pragma unroll
