@@ -100,7 +100,9 @@ __device__ __forceinline__ void push_ghost_images(T* __restrict__ arena, const C
 // flight: the fill of 32,768 blocks of 16^3 takes 470 us, one entry at a time
 // 660.  All index arithmetic is 32 bit, two divisions an entry; with 64-bit
 // divisions in every dimension it took 1650 us, three and a half heat steps.
-template <int D, class T>
+// Index: 64 bit for blocks of more than 2^28 ghost entries, whose numbers and
+// the strides beyond them could pass 32.
+template <int D, class T, class Index>
 __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, CartTopo topo, SlabLayout L,
                                                         int field) {
     constexpr int NS = D == 1 ? 3 : (D == 2 ? 9 : 27);
@@ -110,7 +112,7 @@ __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, C
     const int n0 = topo.n[0], n1 = D > 1 ? topo.n[1] : 1, n2 = D > 2 ? topo.n[2] : 1;
     const int G0 = L.gdim[0], G1 = D > 1 ? L.gdim[1] : 1;
     const int gy = D > 1 ? g : 0, gz = D > 2 ? g : 0;
-    const unsigned first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
+    const Index first = blockIdx.y * blockDim.x + threadIdx.x, stride = gridDim.y * blockDim.x;
     for (int b = blockIdx.x; b < topo.nblocks; b += gridDim.x) {
         __syncthreads();  // the tables of the previous block are no longer read
         if (threadIdx.x < NS) {
@@ -149,33 +151,33 @@ __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, C
         };
         // the entries in one sequence: x ghosts of the interior rows (2 g a
         // row), rows with y outside and z inside, planes with z outside
-        const unsigned per = 2u * g, xs = (unsigned)n1 * n2 * per;
-        const unsigned strip = D > 1 ? 2u * g * G0 : 1, ys = D > 1 ? xs + strip * n2 : xs;
-        const unsigned plane = D > 2 ? (unsigned)G0 * G1 : 1, all = D > 2 ? ys + plane * 2u * g : ys;
-        auto entry = [&](unsigned k, int64_t& to, int64_t& from) {
+        const Index per = 2u * g, xs = (Index)n1 * n2 * per;
+        const Index strip = D > 1 ? (Index)2 * g * G0 : 1, ys = D > 1 ? xs + strip * n2 : xs;
+        const Index plane = D > 2 ? (Index)G0 * G1 : 1, all = D > 2 ? ys + plane * 2u * g : ys;
+        auto entry = [&](Index k, int64_t& to, int64_t& from) {
             if (k < xs) {
-                const unsigned row = k / per, i = k - row * per;
-                const unsigned z = row / n1, y = row - z * n1;
+                const Index row = k / per, i = k - row * per;
+                const Index z = row / n1, y = row - z * n1;
                 place((int)i < g ? (int)i - g : n0 + (int)i - g, (int)y, (int)z, to, from);
             } else if (D > 1 && k < ys) {
                 k -= xs;
-                const unsigned z = k / strip, q = k - z * strip;
-                const unsigned r = q / G0, x = q - r * G0;
+                const Index z = k / strip, q = k - z * strip;
+                const Index r = q / G0, x = q - r * G0;
                 place((int)x - g, (int)r < g ? (int)r - g : n1 + (int)r - g, (int)z, to, from);
             } else if (D > 2) {
                 k -= ys;
-                const unsigned p = k / plane, q = k - p * plane;
-                const unsigned r = q / G0, x = q - r * G0;
+                const Index p = k / plane, q = k - p * plane;
+                const Index r = q / G0, x = q - r * G0;
                 place((int)x - g, (int)r - g, (int)p < g ? (int)p - g : n2 + (int)p - g, to, from);
             }
         };
         constexpr int U = 4;  // entries in flight a thread
-        for (unsigned k = first; k < all; k += U * stride) {
+        for (Index k = first; k < all; k += U * stride) {
             int64_t to[U];
             T v[U];
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const unsigned e = k + u * stride;
+                const Index e = k + u * stride;
                 if (e < all) {
                     int64_t from = 0;
                     entry(e, to[u], from);
@@ -384,17 +386,26 @@ cudaError_t launch_halo_fill(void* arena, int elem_size, const CartTopo& topo, c
     }
     const dim3 grid((unsigned)topo.nblocks,
                     (unsigned)std::max<int64_t>(1, std::min<int64_t>((whole - inner) / 2048, 1024)));
-#define LG_HALO(DD)                                                                                          \
-    do {                                                                                                     \
-        if (elem_size == 8)                                                                                  \
-            halo_fill_kernel<DD, double><<<grid, 256, 0, s>>>(static_cast<double*>(arena), topo, L, field); \
-        else                                                                                                 \
-            halo_fill_kernel<DD, float><<<grid, 256, 0, s>>>(static_cast<float*>(arena), topo, L, field);   \
+    const bool large = whole - inner > (int64_t)1 << 28;
+#define LG_HALO_T(DD, T)                                                                                           \
+    do {                                                                                                           \
+        if (large)                                                                                                 \
+            halo_fill_kernel<DD, T, uint64_t><<<grid, 256, 0, s>>>(static_cast<T*>(arena), topo, L, field);        \
+        else                                                                                                       \
+            halo_fill_kernel<DD, T, unsigned><<<grid, 256, 0, s>>>(static_cast<T*>(arena), topo, L, field);        \
+    } while (0)
+#define LG_HALO(DD)                   \
+    do {                              \
+        if (elem_size == 8)           \
+            LG_HALO_T(DD, double);    \
+        else                          \
+            LG_HALO_T(DD, float);     \
     } while (0)
     if (topo.D == 1) LG_HALO(1);
     else if (topo.D == 2) LG_HALO(2);
     else LG_HALO(3);
 #undef LG_HALO
+#undef LG_HALO_T
     return cudaGetLastError();
 }
 
