@@ -1,8 +1,8 @@
 """RungeKutta4 of Model C on grids of more units than one wave holds, where the
 four stages of a step take theirs from the list and leave it reset for the
 next, read the running sum that other units' warps wrote in the stage before,
-and blocks of 126 and 128 columns have their own instantiations: FP64 has the
-oracle's bits, plain and as a graph (needs a GPU)."""
+and blocks of 32, 64, 126, 128 and 256 columns have their own instantiations:
+FP64 has the oracle's bits, plain and as a graph (needs a GPU)."""
 import numpy as np
 import pytest
 
@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 H, STEPS = 0.4, 6
 
 
-@pytest.mark.parametrize("cells,block", [([1764, 1764], [126, 126]), ([1536, 1664], [128, 128]), ([1600, 1500], [100, 75])])
+@pytest.mark.parametrize("cells,block", [([1764, 1764], [126, 126]), ([1536, 1664], [128, 128]),
+                                         ([1600, 1500], [100, 75]), ([1280, 1024], [32, 64]), ([1280, 1088], [64, 34]),
+                                         ([1536, 1280], [256, 160])])
 @pytest.mark.parametrize("orient", [False, True])
 def test_has_the_oracle_bits(sched, orc, cells, block, orient):
     grid = L.CartesianGrid(cells, block, [0.0, 0.0], [H, H])
