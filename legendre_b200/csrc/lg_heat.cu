@@ -5,6 +5,7 @@
 // rk4.rs:40-79), so the results are the reference's bits.
 #include <algorithm>
 #include <atomic>
+#include <type_traits>
 
 #include "lg_common.cuh"
 #include "lg_heat_plan.h"
@@ -27,7 +28,7 @@ struct HeatArgs {
     const double* y;    // kRkB
     const double* aux_in;
     double* aux;        // kRkA
-    int N[3];           // global cells: x, y (1 in 2-D), march dimension
+    int64_t N[3];       // global cells: x, y (1 in 2-D), march dimension
     int n[3];           // block cells in the same order
     int periodic[3];
     int64_t bstr[3];    // elements between neighbouring blocks of a dimension
@@ -40,20 +41,22 @@ struct HeatArgs {
 // source coordinate of a window position: itself, wrapped, or the mirror
 // image (cartesian.rs:439-526); positions that no result depends on are
 // clamped into the domain
-__device__ __forceinline__ int source_coord(int g, int N, int periodic) {
+template <class Coord>
+__device__ __forceinline__ Coord source_coord(Coord g, Coord N, int periodic) {
     if (periodic) {
         while (g < 0) g += N;
         while (g >= N) g -= N;
         return g;
     }
     if (g < 0) g = -1 - g;
-    if (g >= N) g = 2 * N - 1 - g;
-    return min(max(g, 0), N - 1);
+    if (g >= N) g = N - 1 - (g - N);
+    return min(max(g, (Coord)0), N - 1);
 }
 
 // element offset of global coordinate g of dimension d inside an arena
-__device__ __forceinline__ int64_t coord_offset(const HeatArgs& a, int d, int g) {
-    const int b = g / a.n[d];
+template <class Coord>
+__device__ __forceinline__ int64_t coord_offset(const HeatArgs& a, int d, Coord g) {
+    const Coord b = g / a.n[d];
     return (int64_t)b * a.bstr[d] + (int64_t)(g - b * a.n[d] + 1) * a.cstr[d];
 }
 
@@ -101,11 +104,13 @@ struct MarchTile {
 // The march is unrolled six times, so that the planes in registers, those of
 // the first stage (three) and the double buffers keep their places and
 // nothing is moved (rolled: 90 instead of 53 instructions per cell and
-// step).  Off: the type of a column's byte offset inside one layer of blocks.
+// step).  Off: the type of a column's byte offset inside one layer of blocks and,
+// signed, of a cell's coordinate.
 template <int FORM, int WX, int TR, int R, int PITCH, int MINB, class Off>
 __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, MINB)
     heat_march_kernel(const __grid_constant__ HeatArgs a) {
     using G = MarchTile<FORM, WX, TR, R, PITCH>;
+    using Coord = std::make_signed_t<Off>;
     constexpr bool HASY = G::kHasY;
     constexpr int H = G::kH, WY = G::kWY, PF = G::kAhead, UR = 6;
     __shared__ double A[2][G::kPlane];
@@ -116,43 +121,46 @@ __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, M
     const int cx = t % WX, ty = t / WX;
     const bool thread_in = ty < TR;
     const int wy0 = min(ty, TR - 1) * R;  // idle threads shadow the last rows
+    const Coord NX = (Coord)a.N[0], NY = (Coord)a.N[1], NZ = (Coord)a.N[2];
     int item = blockIdx.x;
-    const int tx0 = (item % a.tiles_x) * G::kOX;
+    const Coord tx0 = (Coord)(item % a.tiles_x) * G::kOX;
     item /= a.tiles_x;
-    const int ty0 = HASY ? (item % a.tiles_y) * G::kOY : 0;
-    const int z0 = (HASY ? item / a.tiles_y : item) * a.zc;
-    const int z1 = min(z0 + a.zc, a.N[2]);
+    const Coord ty0 = HASY ? (Coord)(item % a.tiles_y) * G::kOY : 0;
+    const Coord z0 = (Coord)(HASY ? item / a.tiles_y : item) * a.zc;
+    const Coord z1 = min(z0 + a.zc, NZ);
 
-    const int gx = tx0 - H + cx;
-    const int64_t ox = coord_offset(a, 0, source_coord(gx, a.N[0], a.periodic[0]));
+    const Coord gx = tx0 - H + cx;
+    const int64_t ox = coord_offset(a, 0, source_coord(gx, NX, a.periodic[0]));
     Off base[R];  // bytes
     bool store[R];
-    const bool x_out = thread_in && cx >= H && cx < WX - H && gx < a.N[0];
+    const bool x_out = thread_in && cx >= H && cx < WX - H && gx < NX;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
         int64_t e = ox;
         store[r] = x_out;
         if (HASY) {
-            const int wy = wy0 + r, gy = ty0 - H + wy;
-            e += coord_offset(a, 1, source_coord(gy, a.N[1], a.periodic[1]));
-            store[r] = x_out && wy >= H && wy < WY - H && gy < a.N[1];
+            const int wy = wy0 + r;
+            const Coord gy = ty0 - H + wy;
+            e += coord_offset(a, 1, source_coord(gy, NY, a.periodic[1]));
+            store[r] = x_out && wy >= H && wy < WY - H && gy < NY;
         }
         base[r] = (Off)(e * 8);
     }
     // which of this thread's neighbours are mirror ghosts (second stage only)
-    const bool mxlo = !a.periodic[0] && gx == 0, mxhi = !a.periodic[0] && gx == a.N[0] - 1;
-    int mrow_lo = -1, mrow_hi = -1;
+    const bool mxlo = !a.periodic[0] && gx == 0, mxhi = !a.periodic[0] && gx == NX - 1;
+    Coord mrow_lo = -1, mrow_hi = -1;
     if (HASY && !a.periodic[1]) {
         mrow_lo = H - ty0 - wy0;               // the r whose row is the first one
-        mrow_hi = a.N[1] - 1 + H - ty0 - wy0;  // the r whose row is the last one
+        mrow_hi = NY - 1 + H - ty0 - wy0;  // the r whose row is the last one
     }
     // ghost columns beside a block's first and last column
-    const int ix = gx >= 0 && gx < a.N[0] ? gx % a.n[0] : 1;
+    const int ix = gx >= 0 && gx < NX ? (int)(gx % a.n[0]) : 1;
     const bool glo = x_out && ix == 0, ghi = x_out && ix == a.n[0] - 1;
     // plane offsets; those past the last plane needed stay valid addresses
-    const int pend = z1 + H;
-    for (int k = t; k < z1 - z0 + 2 * H + PF + 1; k += G::kThreads)
-        plane_off[k] = coord_offset(a, 2, source_coord(z0 - H + k, a.N[2], a.periodic[2])) * 8;
+    const Coord pend = z1 + H;
+    const int planes = (int)(z1 - z0);
+    for (int k = t; k < planes + 2 * H + PF + 1; k += G::kThreads)
+        plane_off[k] = coord_offset(a, 2, source_coord(z0 - H + k, NZ, a.periodic[2])) * 8;
     const bool edge =
         __syncthreads_or(mxlo || mxhi || (mrow_lo >= 0 && mrow_lo < R) || (mrow_hi >= 0 && mrow_hi < R)) != 0;
     auto at = [](const double* p, int64_t plane, Off o) {
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, M
         return acc * a.kappa;
     };
 
-    int p = z0 - H;
+    Coord p = z0 - H;
     for (;;) {
 #pragma unroll
         for (int ph = 0; ph < UR; ++ph, ++p, ++po) {
@@ -242,7 +250,7 @@ __global__ void __launch_bounds__(MarchTile<FORM, WX, TR, R, PITCH>::kThreads, M
             } else {
                 // second stage, plane p - 2 (the first stage's rows are in B[e])
                 const double* s = B[e] + sidx;
-                const bool zlo = !a.periodic[2] && p == 2, zhi = !a.periodic[2] && p - 2 == a.N[2] - 1;
+                const bool zlo = !a.periodic[2] && p == 2, zhi = !a.periodic[2] && p - 2 == NZ - 1;
                 const bool in = p - 2 >= z0;
                 const int64_t off = in ? po[-2] : 0;
 #pragma unroll
@@ -310,8 +318,8 @@ template <int FORM, class Off, int WX, int TR, int R, int PITCH, int MINB>
 struct March {
     using G = MarchTile<FORM, WX, TR, R, PITCH>;
     static void tiles(HeatArgs& a) {
-        a.tiles_x = (a.N[0] + G::kOX - 1) / G::kOX;
-        a.tiles_y = (a.N[1] + G::kOY - 1) / G::kOY;
+        a.tiles_x = (int)((a.N[0] + G::kOX - 1) / G::kOX);
+        a.tiles_y = (int)((a.N[1] + G::kOY - 1) / G::kOY);
     }
     static cudaError_t consider(int tile, double factor, HeatArgs a, HeatPlan& plan) {
         int per_sm = 0;
@@ -383,8 +391,10 @@ cudaError_t launch_form(int D, const HeatArgs& a, HeatPlan& plan, cudaStream_t s
 
 template <int FORM>
 cudaError_t launch_form(int D, const HeatArgs& a, HeatPlan& plan, cudaStream_t s) {
-    // a column's byte offset inside one layer of blocks: 32 bits where they hold it
-    return a.bstr[2] < (int64_t)1 << 28 ? launch_form<FORM, uint32_t>(D, a, plan, s)
+    // a column's byte offset inside one layer of blocks, and coordinates two
+    // cells beyond the grid: 32 bits where they hold them
+    const bool small = a.bstr[2] < (int64_t)1 << 28 && std::max({a.N[0], a.N[1], a.N[2]}) < (int64_t)1 << 30;
+    return small ? launch_form<FORM, uint32_t>(D, a, plan, s)
                                        : launch_form<FORM, int64_t>(D, a, plan, s);
 }
 
@@ -405,7 +415,7 @@ HeatArgs march_args(const CartTopo& topo, const SlabLayout& L, int field, const 
             bs *= topo.nb[e];
             cs *= L.gdim[e];
         }
-        a.N[k] = topo.n[d] * topo.nb[d];
+        a.N[k] = (int64_t)topo.n[d] * topo.nb[d];
         a.n[k] = topo.n[d];
         a.periodic[k] = periodic[d];
         a.bstr[k] = bs;
@@ -417,12 +427,7 @@ HeatArgs march_args(const CartTopo& topo, const SlabLayout& L, int field, const 
 }
 }  // namespace
 
-bool heat_march_supported(const CartTopo& topo, const SlabLayout& L) {
-    if ((topo.D != 2 && topo.D != 3) || L.ghost != 1) return false;
-    for (int d = 0; d < topo.D; ++d)
-        if ((int64_t)topo.n[d] * topo.nb[d] > (int64_t)1 << 30) return false;
-    return true;
-}
+bool heat_march_supported(const CartTopo& topo, const SlabLayout& L) { return topo.D >= 2 && L.ghost == 1; }
 
 cudaError_t launch_heat_march_fe(int steps, const double* in, double* out, const CartTopo& topo, const SlabLayout& L,
                                  int field, const int periodic[3], double kappa, double dt, const double inv_h2[3],

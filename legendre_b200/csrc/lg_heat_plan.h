@@ -15,12 +15,12 @@ constexpr int kMaxPlanes = 256;  // planes a CTA marches over, at most
 // sqrt(planes) heights, 256 in all, and once a run: one chunk count after the
 // other at every launch took 5 us on 1425 x 1001, where a launch takes 10.7,
 // and 165 on 128 x 100000.
-inline int march_planes(int64_t tiles, int planes, int halo, int64_t slots) {
+inline int march_planes(int64_t tiles, int64_t planes, int halo, int64_t slots) {
     int64_t best = -1;
-    int best_zc = std::min(planes, kMaxPlanes);
+    int best_zc = (int)std::min<int64_t>(planes, kMaxPlanes);
     for (int zc = best_zc; zc >= 1; --zc) {
-        const unsigned chunks = ((unsigned)planes + zc - 1) / zc;
-        zc = (int)(((unsigned)planes + chunks - 1) / chunks);  // the lowest height with as many chunks
+        const int64_t chunks = (planes + zc - 1) / zc;
+        zc = (int)((planes + chunks - 1) / chunks);  // the lowest height with as many chunks
         const int64_t ctas = tiles * chunks;
         const int64_t cost = (ctas + slots - 1) / slots * (zc + 2 * halo + 4);
         if (best < 0 || cost < best) {
@@ -39,8 +39,8 @@ inline int march_planes(int64_t tiles, int planes, int halo, int64_t slots) {
 // Forward Euler on cubes of 40^3 to 400^3 and on narrow grids (4 to 33 cells in
 // one or two dimensions): the cheapest shape by this is the fastest one or
 // within 4 %, 9 % at 4096 x 8 x 8; RungeKutta4 within 5 %.
-inline double march_cost(int64_t tiles, int planes, int zc, int halo, int64_t sms, int per_sm, int threads, int rows) {
-    const int64_t ctas = tiles * (((int64_t)planes + zc - 1) / zc), slots = sms * per_sm;
+inline double march_cost(int64_t tiles, int64_t planes, int zc, int halo, int64_t sms, int per_sm, int threads, int rows) {
+    const int64_t ctas = tiles * ((planes + zc - 1) / zc), slots = sms * per_sm;
     const int64_t share = std::min<int64_t>(per_sm, (ctas + sms - 1) / sms);
     return (double)((ctas + slots - 1) / slots) * (zc + 2 * halo + 4) *
            std::max(1000.0, (double)share * threads * (rows + 0.5));

@@ -191,39 +191,31 @@ __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, C
     }
 }
 
-// ------------------------------------------------------------- heat (d) --
-// Heat<D>::vector_field_block (examples/heat3d.rs:63-79): the central
+// --------------------------------------------------- heat in 1-D (d) --
+// Heat<1>::vector_field_block (examples/heat3d.rs:63-79): the central
 // Laplacian (finite_difference.rs:49-67) times kappa, then ForwardEuler's
 // axpy (integrators/euler.rs:51-53).  One thread per interior cell.
-template <int D>
+__device__ __forceinline__ double heat_drift_1d(const double* s, int64_t o, double kappa, double ih) {
+    const double center = s[o];
+    double acc = 0.0;
+    acc += ((s[o + 1] - (center + center)) + s[o - 1]) * ih;
+    return acc * kappa;
+}
+
 __global__ void __launch_bounds__(256) heat_step_kernel(const double* __restrict__ in, double* __restrict__ out,
                                                         CartTopo topo, SlabLayout L, int field, double kappa,
-                                                        double dt, double ih0, double ih1, double ih2) {
-    const int64_t cells = (int64_t)topo.n[0] * (D > 1 ? topo.n[1] : 1) * (D > 2 ? topo.n[2] : 1);
-    const int64_t st1 = L.gdim[0];
-    const int64_t st2 = (int64_t)L.gdim[0] * (D > 1 ? L.gdim[1] : 1);
+                                                        double dt, double ih) {
     for (int b = blockIdx.y; b < topo.nblocks; b += gridDim.y) {
-    const double* s = in + slab_base(L, b, field);
-    double* o_slab = out + slab_base(L, b, field);
-    for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cells;
-         c += (int64_t)gridDim.x * blockDim.x) {
-        int l[3] = {0, 0, 0};
-        int64_t rem = c;
-        l[0] = (int)(rem % topo.n[0]);
-        rem /= topo.n[0];
-        if (D > 1) { l[1] = (int)(rem % topo.n[1]); rem /= topo.n[1]; }
-        if (D > 2) l[2] = (int)rem;
-        const int64_t o = lin<D>(L, l);
-        const double center = s[o];
-        double acc = 0.0;
-        acc += ((s[o + 1] - (center + center)) + s[o - 1]) * ih0;
-        if (D > 1) acc += ((s[o + st1] - (center + center)) + s[o - st1]) * ih1;
-        if (D > 2) acc += ((s[o + st2] - (center + center)) + s[o - st2]) * ih2;
-        const double k = acc * kappa;
-        const double v = center + dt * k;
-        o_slab[o] = v;
-        push_ghost_images<D, double>(out, topo, L, field, b, l, v);
-    }
+        const int64_t base = slab_base(L, b, field);
+        const double* s = in + base;
+        for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < topo.n[0];
+             c += (int64_t)gridDim.x * blockDim.x) {
+            const int l[1] = {(int)c};
+            const int64_t o = lin<1>(L, l);
+            const double v = s[o] + dt * heat_drift_1d(s, o, kappa, ih);
+            out[base + o] = v;
+            push_ghost_images<1, double>(out, topo, L, field, b, l, v);
+        }
     }
 }
 
@@ -232,35 +224,20 @@ __global__ void __launch_bounds__(256) heat_step_kernel(const double* __restrict
 //   MODE 1: kout = k, out = y + c k          (y_tmp = y; y_tmp += c k_i)
 //   MODE 2: out = (((y + s6 k1) + s3 k2) + s3 k3) + s6 k   (the four axpys)
 // with the output's ghost images pushed for the next stage.
-template <int D, int MODE>
+template <int MODE>
 __global__ void __launch_bounds__(256) heat_rk_kernel(const double* __restrict__ in, double* __restrict__ out,
                                                       const double* __restrict__ y, double* __restrict__ kout,
                                                       const double* __restrict__ k1, const double* __restrict__ k2,
                                                       const double* __restrict__ k3, CartTopo topo, SlabLayout L,
-                                                      int field, double kappa, double ih0, double ih1, double ih2,
-                                                      double c, double s6, double s3) {
-    const int64_t cells = (int64_t)topo.n[0] * (D > 1 ? topo.n[1] : 1) * (D > 2 ? topo.n[2] : 1);
-    const int64_t st1 = L.gdim[0];
-    const int64_t st2 = (int64_t)L.gdim[0] * (D > 1 ? L.gdim[1] : 1);
+                                                      int field, double kappa, double ih, double c, double s6,
+                                                      double s3) {
     for (int b = blockIdx.y; b < topo.nblocks; b += gridDim.y) {
         const int64_t base = slab_base(L, b, field);
-        const double* s = in + base;
-        for (int64_t cc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cc < cells;
+        for (int64_t cc = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; cc < topo.n[0];
              cc += (int64_t)gridDim.x * blockDim.x) {
-            int l[3] = {0, 0, 0};
-            int64_t rem = cc;
-            l[0] = (int)(rem % topo.n[0]);
-            rem /= topo.n[0];
-            if (D > 1) { l[1] = (int)(rem % topo.n[1]); rem /= topo.n[1]; }
-            if (D > 2) l[2] = (int)rem;
-            const int64_t o = lin<D>(L, l);
-            const double center = s[o];
-            double acc = 0.0;
-            acc += ((s[o + 1] - (center + center)) + s[o - 1]) * ih0;
-            if (D > 1) acc += ((s[o + st1] - (center + center)) + s[o - st1]) * ih1;
-            if (D > 2) acc += ((s[o + st2] - (center + center)) + s[o - st2]) * ih2;
-            const double k = acc * kappa;
-            const int64_t e = base + o;
+            const int l[1] = {(int)cc};
+            const int64_t o = lin<1>(L, l), e = base + o;
+            const double k = heat_drift_1d(in + base, o, kappa, ih);
             double v;
             if (MODE == 1) {
                 kout[e] = k;
@@ -273,7 +250,7 @@ __global__ void __launch_bounds__(256) heat_rk_kernel(const double* __restrict__
                 v = v + s6 * k;
             }
             out[e] = v;
-            push_ghost_images<D, double>(out, topo, L, field, b, l, v);
+            push_ghost_images<1, double>(out, topo, L, field, b, l, v);
         }
     }
 }
@@ -413,40 +390,21 @@ cudaError_t launch_heat_rk_stage(int mode, const double* in, double* out, const 
                                  const double* k1, const double* k2, const double* k3, const CartTopo& topo,
                                  const SlabLayout& L, int field, double kappa, const double* inv_h2, double c,
                                  double s6, double s3, cudaStream_t s) {
-    const int64_t cells = (int64_t)topo.n[0] * (topo.D > 1 ? topo.n[1] : 1) * (topo.D > 2 ? topo.n[2] : 1);
-    const dim3 grid((unsigned)std::min<int64_t>((cells + 255) / 256, 1024), (unsigned)std::min(topo.nblocks, 65535));
-#define LG_HRK(DD, MM)                                                                                             \
-    heat_rk_kernel<DD, MM><<<grid, 256, 0, s>>>(in, out, y, kout, k1, k2, k3, topo, L, field, kappa, inv_h2[0],   \
-                                                 inv_h2[1], inv_h2[2], c, s6, s3)
-    if (mode == 1) {
-        if (topo.D == 1) LG_HRK(1, 1);
-        else if (topo.D == 2) LG_HRK(2, 1);
-        else LG_HRK(3, 1);
-    } else {
-        if (topo.D == 1) LG_HRK(1, 2);
-        else if (topo.D == 2) LG_HRK(2, 2);
-        else LG_HRK(3, 2);
-    }
-#undef LG_HRK
+    if (topo.D != 1) return cudaErrorInvalidValue;
+    const dim3 grid((unsigned)std::min<int64_t>(((int64_t)topo.n[0] + 255) / 256, 1024),
+                    (unsigned)std::min(topo.nblocks, 65535));
+    if (mode == 1)
+        heat_rk_kernel<1><<<grid, 256, 0, s>>>(in, out, y, kout, k1, k2, k3, topo, L, field, kappa, inv_h2[0], c, s6, s3);
+    else
+        heat_rk_kernel<2><<<grid, 256, 0, s>>>(in, out, y, kout, k1, k2, k3, topo, L, field, kappa, inv_h2[0], c, s6, s3);
     return cudaGetLastError();
 }
 
 cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
                              double kappa, double dt, const double inv_h2[3], cudaStream_t s) {
-    int64_t cells = 1;
-    for (int d = 0; d < topo.D; ++d) cells *= topo.n[d];
-    dim3 grid(grid_x_for(cells, 256), grid_y_for(topo.nblocks));
-    switch (topo.D) {
-        case 1:
-            heat_step_kernel<1><<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0], 0.0, 0.0);
-            break;
-        case 2:
-            heat_step_kernel<2><<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0], inv_h2[1], 0.0);
-            break;
-        default:
-            heat_step_kernel<3><<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0], inv_h2[1],
-                                                     inv_h2[2]);
-    }
+    if (topo.D != 1) return cudaErrorInvalidValue;
+    dim3 grid(grid_x_for(topo.n[0], 256), grid_y_for(topo.nblocks));
+    heat_step_kernel<<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0]);
     return cudaGetLastError();
 }
 

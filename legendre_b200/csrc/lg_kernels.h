@@ -33,7 +33,7 @@ cudaError_t launch_halo_fill(void* arena, int elem_size, const CartTopo& topo, c
 
 // (d) forward-Euler heat step: out = in + dt * (kappa * lap(in)) on the
 // interiors, plus the ghost ring of `out` filled from the new interiors.  1-D
-// grids (and dimensions of more than 2^30 cells); the others march (below).
+// grids; the others march (below).
 cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
                              double kappa, double dt, const double inv_h2[3], cudaStream_t s);
 
@@ -75,7 +75,7 @@ cudaError_t launch_modelc_step_f32(const float* in, float* out, const CartTopo& 
 // One RungeKutta4 stage of the heat model (rk4.rs:40-79): mode 1 writes
 // k = kappa lap(in) to kout and y + c k to out; mode 2 writes
 // (((y + s6 k1) + s3 k2) + s3 k3) + s6 k to out.  Ghost images of out are
-// pushed.  FP64, any dimension, bit-identical to the reference's stages.
+// pushed.  FP64, 1-D, bit-identical to the reference's stages.
 cudaError_t launch_heat_rk_stage(int mode, const double* in, double* out, const double* y, double* kout,
                                  const double* k1, const double* k2, const double* k3, const CartTopo& topo,
                                  const SlabLayout& L, int field, double kappa, const double* inv_h2, double c,
