@@ -47,6 +47,7 @@
 
 #include "lg_common.cuh"
 #include "lg_kernels.h"
+#include "lg_strip_plan.h"
 #include "lg_modelc_ops.cuh"
 
 namespace lg {
@@ -847,14 +848,13 @@ constexpr int strip_group() {
 // unit: 64^2 4.8, 6.8, 11.0, 19.4 us a step; 512^2 8.6, 8.4, 11.2, 19.5; 1008^2
 // 25.0, 21.2, 19.8, 25.1; 2048^2 98, 77, 67, 63.
 //
-// FP32 multi-grain and batched (TAILED): a single wave runs as fast as its units, but from
+// FP32 multi-grain (TAILED): a single wave runs as fast as its units, but from
 // one wave on half a unit's time is spent on the last, partly filled one, so
 // heights between the powers of two pay.  With noise at 6, 8, 12, 16, 32 rows:
 // 500^2 in blocks of 100^2 9.4, 11.3, 10.5, 12.5, 21.6 us a step; 1500^2 50.3,
 // 47.5, 46.8, 53.2, 63.1; 2520^2 (126^2) 95.7, 91.0, 89.5, 84.8, 92.3.  Within
 // 1 % of the best height on average over 500^2 to 3072^2, 7 % at most; the
-// rule above chose up to 30 % off.  48 instances of 144^2 in blocks of 48^2
-// 25.0 -> 24.1 us a step.
+// rule above chose up to 30 % off.
 template <class T, bool TAILED>
 inline int strip_auto_rows(const CartTopo& topo, int strips, int64_t slots) {
     const int n1 = topo.n[1];
@@ -922,7 +922,10 @@ inline dim3 strip_ctas(const TileArgs& g, int ctas_per_sm) {
 // PAIR: the paired rows (256 instances of 256^2, FP32: 102.5 against 79.8 Gcell/s)
 template <class T, class Ops, bool NOISE, int MINB, bool PAIR = false>
 cudaError_t launch_strip_batch(const T* in, T* out, TileArgs g, BatchArgs bt, T dt, T scale_amp, cudaStream_t s) {
-    const bool tail = strip_plan<T, sizeof(T) == 4>(g, strip_group<T, false, PAIR>(), MINB);
+    constexpr bool kFixed = sizeof(T) == 4;
+    if (kFixed && g.rows <= 0)
+        g.rows = strip_batch_rows_f32(g.topo.nblocks, (g.topo.n[0] + 31) / 32, g.topo.n[1], device_sm_count());
+    const bool tail = strip_plan<T>(g, kFixed ? 4 : strip_group<T, false, PAIR>(), MINB);
     const dim3 grid = strip_ctas(g, MINB);
     const typename Ops::Params m{};
     if (tail) {

@@ -1,6 +1,6 @@
-"""FP32 multi-grain and batched steps at the unit heights their plan chooses
-(6, 10, 12, 20 and 24 rows beside the powers of two; blocks that no height
-divides): every height has the values of the two-row units, within the few
+"""FP32 multi-grain steps at the unit heights their plan chooses (6, 10, 12, 20
+and 24 rows beside the powers of two; blocks that no height divides), and
+batches at theirs: every height has the values of the two-row units, within the few
 rounding steps by which the units' first faces may be contracted differently
 (needs a GPU)."""
 import numpy as np
