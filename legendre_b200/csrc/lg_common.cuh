@@ -98,31 +98,26 @@ __device__ __forceinline__ double log_unit_interval(double n) {
 // cos: x = k pi/2 + r, |r| <= pi/4, with pi/2 in two parts (the first
 // subtraction is exact), then the sine r + r z S(z) or the cosine 1 + z C(z),
 // z = r^2, and the quadrant's sign.  S and C minimise the relative error on
-// that interval (Remez exchange; 3.6e-18 and 5.6e-20).  Both are evaluated: a
-// warp's lanes draw all quadrants.  One polynomial over |r| <= pi/2 takes six
-// fmas less (10080^2 4 % faster with a root within an ulp), but its rounding
-// errors are larger: the Gaussian's mean error 8.0e-17 against 7.5e-17.
+// that interval (Remez exchange; 3.6e-18 and 5.6e-20).  A warp's lanes draw all
+// quadrants, so the coefficients are selected (two polynomials and a select of
+// the results run 10080^2 1.6 % and blocks of 196 x 146 3 % slower, by spills).
+// One polynomial over |r| <= pi/2 takes fewer instructions (10080^2 4 % faster
+// with a root within an ulp), but its rounding errors are larger: the
+// Gaussian's mean error 8.0e-17 against 7.5e-17.
 __device__ __forceinline__ double cos_full_turn(double x, int top) {
     const int k = (top + 1) >> 1;
     const double kd = __hiloint2double(0x43300000, k) - 0x1p52;
     const double r = fma(-kd, 0x1.1a62633145c07p-54, fma(-kd, 0x1.921fb54442d18p+0, x));
     const double z = r * r;
-    double s = 0x1.5d8fba92fea51p-33;
-    s = fma(s, z, -0x1.ae5e5a4426ab5p-26);
-    s = fma(s, z, 0x1.71de3567738e7p-19);
-    s = fma(s, z, -0x1.a01a019bfd844p-13);
-    s = fma(s, z, 0x1.111111110f7cdp-7);
-    s = fma(s, z, -0x1.5555555555548p-3);
-    s = fma(r * z, s, r);
-    double c = -0x1.8fa4800fb4bcbp-37;
-    c = fma(c, z, 0x1.1ee9d783e31abp-29);
-    c = fma(c, z, -0x1.27e4f7ea7e667p-22);
-    c = fma(c, z, 0x1.a01a019c83f08p-16);
-    c = fma(c, z, -0x1.6c16c16c14f8ep-10);
-    c = fma(c, z, 0x1.555555555554bp-5);
-    c = fma(c, z, -0.5);
-    c = fma(z, c, 1.0);
-    const double v = (k & 1) ? s : c;
+    const bool odd = k & 1;
+    double q = odd ? 0.0 : -0x1.8fa4800fb4bcbp-37;
+    q = fma(q, z, odd ? 0x1.5d8fba92fea51p-33 : 0x1.1ee9d783e31abp-29);
+    q = fma(q, z, odd ? -0x1.ae5e5a4426ab5p-26 : -0x1.27e4f7ea7e667p-22);
+    q = fma(q, z, odd ? 0x1.71de3567738e7p-19 : 0x1.a01a019c83f08p-16);
+    q = fma(q, z, odd ? -0x1.a01a019bfd844p-13 : -0x1.6c16c16c14f8ep-10);
+    q = fma(q, z, odd ? 0x1.111111110f7cdp-7 : 0x1.555555555554bp-5);
+    q = fma(q, z, odd ? -0x1.5555555555548p-3 : -0.5);
+    const double v = fma(odd ? r * z : z, q, odd ? r : 1.0);
     return __hiloint2double(__double2hiint(v) ^ (((k + 1) & 2) << 30), __double2loint(v));
 }
 
