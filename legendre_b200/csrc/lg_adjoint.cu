@@ -844,11 +844,12 @@ int adjoint_strips(const Geo& g) { return (g.N0 + SW - 1) / SW; }
 // starting, and a row takes the same time until the resident warps are all
 // busy; from there on the units queue.  FP32: halved while the launch would
 // hold fewer units than 15 warps per SM, most of one wave of 16 (down to 16
-// rows).  There the contracted sums of a unit's first rows round as they do
-// nowhere else, so moving the boundaries moves the gradients' last bits (2e-8
-// relative); 8-row units would run 32 instances of 128^2 in 24.5 instead of
-// 28 us a step.  On 256 instances of 256^2 whole instances (2304 units, 97 %
-// of a wave) are best.
+// rows).  Other heights move its results by 1e-8 of their size: the parameter
+// gradients because a lane's partial sums, in FP32, then hold other rows, and a
+// few cells' cotangents (33 of 262144 with 8 rows for 16) because the first
+// rows of a unit are contracted otherwise than those inside it.  8-row units
+// would run 32 instances of 128^2 in 24.5 instead of 28 us a step.  On 256
+// instances of 256^2 whole instances (2304 units, 97 % of a wave) are best.
 int adjoint_strip_rows(int dtype, const Geo& g) {
     const int strips = adjoint_strips(g);
     if (dtype != 0) {
