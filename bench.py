@@ -74,13 +74,13 @@ BYTES_PER_CELL = {"f64": 32, "f32": 16}  # read phi, u; write phi, u
 # ncu capture each of the kernel as it now is (the summaries under
 # profiles/ named in NCU_INST): the FP64 and FP32 strip kernels in the
 # variant the autotuner picks on 10080^2 (CAPTURED_VARIANT), captured on
-# 5040^2 of the same 126^2 blocks (808.3 MB and 376.9 MB per 25.4M-cell
-# launch), and the marching heat kernel on 256^3 (292.9 MB per launch of two
-# steps of 16.8M cells).  Traffic grows with the cell
+# 5040^2 of the same 126^2 blocks (808.9 MB and 377.4 MB per 25.4M-cell
+# launch), and the marching heat kernel on 320^3 (593.4 MB per launch of two
+# steps of 32.8M cells).  Traffic grows with the cell
 # count, so a launch of the full grid moves the per-cell figure times its
 # cells.  Other workloads report null.
-TRAFFIC_PER_CELL = {("c3", "f64"): 808.3e6 / 5040 ** 2, ("c3", "f32"): 376.9e6 / 5040 ** 2,
-                    ("c1big", "f64"): 292.9e6 / (2 * 256 ** 3)}
+TRAFFIC_PER_CELL = {("c3", "f64"): 808.9e6 / 5040 ** 2, ("c3", "f32"): 377.4e6 / 5040 ** 2,
+                    ("c1big", "f64"): 593.4e6 / (2 * 320 ** 3)}
 
 NOMINAL_HBM_GBS = 8000.0  # a B200's nominal HBM3e bandwidth, the second denominator
 
@@ -88,12 +88,12 @@ NOMINAL_HBM_GBS = 8000.0  # a B200's nominal HBM3e bandwidth, the second denomin
 # captures (smsp__inst_executed and the fp64 pipe's share, x 32 threads per
 # warp instruction, divided by the launch's cell-updates); the capture named
 # is the summary under profiles/.
-NCU_INST = {("c3", "f64"): {"inst_per_cell": 315.4, "fp64_inst_per_cell": 88.0,
+NCU_INST = {("c3", "f64"): {"inst_per_cell": 337.6, "fp64_inst_per_cell": 91.1,
                             "capture": "modelc_strip_f64_5040sq_126blocks"},
             ("c3", "f32"): {"inst_per_cell": 230.9, "fp64_inst_per_cell": None,
                             "capture": "modelc_strip_f32_5040sq_126blocks"},
-            ("c1big", "f64"): {"inst_per_cell": 63.1, "fp64_inst_per_cell": None,
-                               "capture": "heat_march_256cube"}}
+            ("c1big", "f64"): {"inst_per_cell": 54.7, "fp64_inst_per_cell": None,
+                               "capture": "heat_march_320cube"}}
 
 # the strip-kernel variant the captures ran (the autotuner's choice on 10080^2)
 CAPTURED_VARIANT = 32015
