@@ -138,12 +138,12 @@ int64_t face_neighbor(const lg_grid* g, int64_t b, int dim, int dir) {
     return id;
 }
 
-int fill_all_ghosts(lg_state* st) {
+int fill_all_ghosts(lg_state* st, bool dependent = false) {
     lg_ctx* ctx = st->ctx;
     for (int f = 0; f < st->nfields; ++f) {
         if (st->ghosts[f] == 0) continue;
         cudaError_t e = lg::launch_halo_fill(st->arena[st->cur], st->esize, topo_of(st->grid), layout_of(st, f), f,
-                                             ctx->stream);
+                                             ctx->stream, dependent);
         ctx->launches++;
         if (e != cudaSuccess) return cuda_fail(ctx, e, "halo fill launch");
     }
@@ -570,7 +570,7 @@ int lg_heat_fe_run(lg_state* st, int field, double kappa, double dt, int64_t nst
     if (rc == LG_OK) rc = run_steps(st, key, nsteps - 2 * doubles, flags, [&] { return launch(1); });
     if (rc != LG_OK) return rc;
     if (march && nsteps > 0) {
-        rc = fill_all_ghosts(st);
+        rc = fill_all_ghosts(st, !(flags & LG_RUN_GRAPH));
         if (rc != LG_OK) return rc;
     }
     advance_time(st, dt, nsteps);
@@ -914,7 +914,7 @@ int lg_heat_rk4_run(lg_state* st, int field, double kappa, double dt, int64_t ns
         return LG_OK;
     };
     rc = run_steps(st, key, nsteps, flags, step);
-    if (rc == LG_OK && march && nsteps > 0) rc = fill_all_ghosts(st);
+    if (rc == LG_OK && march && nsteps > 0) rc = fill_all_ghosts(st, !(flags & LG_RUN_GRAPH));
     if (rc != LG_OK) return rc;
     advance_time(st, dt, nsteps);
     return LG_OK;

@@ -28,8 +28,9 @@ struct NoiseDev {
 
 // (b) ghost fill of one field (pull form): every ghost entry of every block
 // copies its source interior entry (exchange, periodic wrap or mirror).
+// `dependent`: launched as dependent on the kernel before it in the stream.
 cudaError_t launch_halo_fill(void* arena, int elem_size, const CartTopo& topo, const SlabLayout& L, int field,
-                             cudaStream_t s);
+                             cudaStream_t s, bool dependent = false);
 
 // (d) forward-Euler heat step: out = in + dt * (kappa * lap(in)) on the
 // interiors, plus the ghost ring of `out` filled from the new interiors.  1-D
