@@ -544,9 +544,13 @@ int lg_heat_fe_run(lg_state* st, int field, double kappa, double dt, int64_t nst
     char key[256];
     snprintf(key, sizeof key, "heat|f=%d|k=%a|dt=%a", field, kappa, dt);
     // 2-D and 3-D: two steps per launch, halos read from the neighbour blocks'
-    // interiors, ghosts filled once at the end; 1-D: the push kernel, one step
-    // per launch, which keeps the ghosts valid
-    const bool march = lg::heat_march_supported(topo, L);
+    // interiors, ghosts filled once at the end.  1-D, and one step of a 2-D grid
+    // of up to 2^19 cells: the kernel of one thread a cell, which keeps the
+    // ghosts valid (one step a call, marched and filled against pushed: 64^2 8.0,
+    // 6.7 us, 512^2 8.3, 6.6, 1000^2 11.2, 13.1)
+    const int64_t grid_cells = st->grid->nblocks * st->grid->block[0] * (topo.D > 1 ? st->grid->block[1] : 1);
+    const bool march = lg::heat_march_supported(topo, L) &&
+                       !(topo.D == 2 && nsteps == 1 && grid_cells <= (int64_t)1 << 19);
     lg::HeatPlan plans[2];
     auto launch = [&](int steps) -> int {
         const double* in = static_cast<const double*>(st->arena[st->cur]);

@@ -198,30 +198,40 @@ __global__ void __launch_bounds__(256) halo_fill_kernel(T* __restrict__ arena, C
     }
 }
 
-// --------------------------------------------------- heat in 1-D (d) --
-// Heat<1>::vector_field_block (examples/heat3d.rs:63-79): the central
+// ------------------------------------ heat, one thread per cell (d) --
+// Heat<D>::vector_field_block (examples/heat3d.rs:63-79): the central
 // Laplacian (finite_difference.rs:49-67) times kappa, then ForwardEuler's
-// axpy (integrators/euler.rs:51-53).  One thread per interior cell.
-__device__ __forceinline__ double heat_drift_1d(const double* s, int64_t o, double kappa, double ih) {
+// axpy (integrators/euler.rs:51-53).  1-D, and single steps of small 2-D grids,
+// which need no fill afterwards.
+template <int D>
+__device__ __forceinline__ double heat_drift(const double* s, int64_t o, int64_t st1, double kappa, double ih0,
+                                             double ih1) {
     const double center = s[o];
     double acc = 0.0;
-    acc += ((s[o + 1] - (center + center)) + s[o - 1]) * ih;
+    acc += ((s[o + 1] - (center + center)) + s[o - 1]) * ih0;
+    if (D > 1) acc += ((s[o + st1] - (center + center)) + s[o - st1]) * ih1;
     return acc * kappa;
 }
 
+template <int D>
 __global__ void __launch_bounds__(256) heat_step_kernel(const double* __restrict__ in, double* __restrict__ out,
                                                         CartTopo topo, SlabLayout L, int field, double kappa,
-                                                        double dt, double ih) {
+                                                        double dt, double ih0, double ih1) {
+    const int64_t cells = (int64_t)topo.n[0] * (D > 1 ? topo.n[1] : 1);
     for (int b = blockIdx.y; b < topo.nblocks; b += gridDim.y) {
         const int64_t base = slab_base(L, b, field);
         const double* s = in + base;
-        for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < topo.n[0];
+        for (int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; c < cells;
              c += (int64_t)gridDim.x * blockDim.x) {
-            const int l[1] = {(int)c};
-            const int64_t o = lin<1>(L, l);
-            const double v = s[o] + dt * heat_drift_1d(s, o, kappa, ih);
+            int l[2] = {(int)c, 0};
+            if (D > 1) {
+                l[1] = (int)(c / topo.n[0]);
+                l[0] = (int)(c - (int64_t)l[1] * topo.n[0]);
+            }
+            const int64_t o = lin<D>(L, l);
+            const double v = s[o] + dt * heat_drift<D>(s, o, L.gdim[0], kappa, ih0, ih1);
             out[base + o] = v;
-            push_ghost_images<1, double>(out, topo, L, field, b, l, v);
+            push_ghost_images<D, double>(out, topo, L, field, b, l, v);
         }
     }
 }
@@ -244,7 +254,7 @@ __global__ void __launch_bounds__(256) heat_rk_kernel(const double* __restrict__
              cc += (int64_t)gridDim.x * blockDim.x) {
             const int l[1] = {(int)cc};
             const int64_t o = lin<1>(L, l), e = base + o;
-            const double k = heat_drift_1d(in + base, o, kappa, ih);
+            const double k = heat_drift<1>(in + base, o, 0, kappa, ih, 0.0);
             double v;
             if (MODE == 1) {
                 kout[e] = k;
@@ -405,9 +415,12 @@ cudaError_t launch_heat_rk_stage(int mode, const double* in, double* out, const 
 
 cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
                              double kappa, double dt, const double inv_h2[3], cudaStream_t s) {
-    if (topo.D != 1) return cudaErrorInvalidValue;
-    dim3 grid(grid_x_for(topo.n[0], 256), grid_y_for(topo.nblocks));
-    heat_step_kernel<<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0]);
+    if (topo.D > 2) return cudaErrorInvalidValue;
+    dim3 grid(grid_x_for((int64_t)topo.n[0] * (topo.D > 1 ? topo.n[1] : 1), 256), grid_y_for(topo.nblocks));
+    if (topo.D == 1)
+        heat_step_kernel<1><<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0], 0.0);
+    else
+        heat_step_kernel<2><<<grid, 256, 0, s>>>(in, out, topo, L, field, kappa, dt, inv_h2[0], inv_h2[1]);
     return cudaGetLastError();
 }
 

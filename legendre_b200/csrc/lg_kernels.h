@@ -34,7 +34,7 @@ cudaError_t launch_halo_fill(void* arena, int elem_size, const CartTopo& topo, c
 
 // (d) forward-Euler heat step: out = in + dt * (kappa * lap(in)) on the
 // interiors, plus the ghost ring of `out` filled from the new interiors.  1-D
-// grids; the others march (below).
+// and 2-D grids; the others, and most 2-D runs, march (below).
 cudaError_t launch_heat_step(const double* in, double* out, const CartTopo& topo, const SlabLayout& L, int field,
                              double kappa, double dt, const double inv_h2[3], cudaStream_t s);
 
